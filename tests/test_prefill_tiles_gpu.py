@@ -1,0 +1,85 @@
+"""Prompt attention at the edges of its 128-query / 128-key tiles, against float64 (GPU).
+
+Probabilities enter as two 16-bit terms (error 2^-16 of a probability or less), sums are fp32, so an output differs from the
+float64 softmax by its own rounding (2^-11 / 2^-8 of its value) and about 2^-15 of the largest value that it averages.
+"""
+
+import pytest
+import torch
+
+from pare_b200.kv_cache import prefill_attention
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, causal, scale):
+    rep, tq, tk = q.shape[1] // k.shape[1], q.shape[2], k.shape[2]
+    s = q.double() @ k.double().repeat_interleave(rep, 1).transpose(-1, -2) * scale
+    if causal:
+        hidden = torch.arange(tk, device="cuda")[None] > torch.arange(tq, device="cuda")[:, None] + tk - tq
+        s = s.masked_fill(hidden, float("-inf"))
+    return torch.softmax(s, -1) @ v.double().repeat_interleave(rep, 1)
+
+
+def _check(b, hq, h, tq, tk, dtype, causal=True, spread=1.0, scale=128 ** -0.5):
+    g = torch.Generator("cuda").manual_seed(tq * 31 + tk)
+    q = (torch.randn(b, hq, tq, 128, device="cuda", generator=g) * spread).to(dtype)
+    k = torch.randn(b, h, tk, 128, device="cuda", generator=g).to(dtype)
+    v = torch.randn(b, h, tk, 128, device="cuda", generator=g).to(dtype)
+    out = prefill_attention(q, k, v, scale=scale, causal=causal)
+    ref = _reference(q, k, v, causal, scale)
+    ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    # 2^-21 of a logit's magnitude (fp32 product and sum) goes into the exponent
+    bound = ulp * ref.abs() + (2.0 ** -15 + 2.0 ** -21 * float((q.double().norm(dim=-1).max() * 12 * scale))) * float(v.abs().max())
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    assert torch.equal(out, prefill_attention(q, k, v, scale=scale, causal=causal))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tq,tk", [(1, 1), (1, 129), (127, 127), (128, 128), (129, 129), (255, 511), (257, 257), (300, 1000), (640, 641)])
+def test_length_edges(tq, tk, dtype, cuda_lib):
+    _check(1, 4, 2, tq, tk, dtype)
+    _check(1, 2, 2, tq, tk, dtype, causal=False)
+
+
+@pytest.mark.parametrize("hq,h", [(1, 1), (3, 1), (7, 1), (14, 2), (5, 5), (16, 2)])
+@pytest.mark.parametrize("t", [100, 260, 400])
+def test_heads_that_share_a_kv_head(hq, h, t, cuda_lib):
+    """Even and odd numbers of query heads per KV head, odd and even numbers of query tiles: every (head, tile) exactly once."""
+    _check(2, hq, h, t, t, torch.float16)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_maximum_that_keeps_growing(dtype, cuda_lib):
+    """Logits with a standard deviation of 12, later keys larger than earlier ones: the running maximum is raised again and again."""
+    g = torch.Generator("cuda").manual_seed(1)
+    t = 700
+    k = torch.randn(1, 1, t, 128, device="cuda", generator=g) * torch.linspace(0.2, 4.0, t, device="cuda")[None, None, :, None]
+    q = torch.randn(1, 2, t, 128, device="cuda", generator=g) * 3.0
+    v = torch.randn(1, 1, t, 128, device="cuda", generator=g)
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    out = prefill_attention(q, k, v)
+    ref = _reference(q, k, v, True, 128 ** -0.5)
+    ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert bool(((out.double() - ref).abs() <= ulp * ref.abs() + 2.0 ** -12 * float(v.abs().max())).all())
+
+
+def test_broadcast_and_negative_scale_take_the_general_path(cuda_lib):
+    """What a tensor map cannot describe (a broadcast batch) and a negative scale: the same results."""
+    g = torch.Generator("cuda").manual_seed(2)
+    q = torch.randn(2, 4, 200, 128, device="cuda", generator=g).half()
+    k = torch.randn(1, 2, 200, 128, device="cuda", generator=g).half().expand(2, 2, 200, 128)
+    v = torch.randn(1, 2, 200, 128, device="cuda", generator=g).half().expand(2, 2, 200, 128)
+    for scale in (128 ** -0.5, -0.1):
+        out = prefill_attention(q, k, v, scale=scale)
+        ref = _reference(q, k, v, True, scale)
+        assert bool(((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -13 * float(v.abs().max())).all())
+
+
+def test_infinite_logit_gives_nan_and_hidden_keys_do_not_matter(cuda_lib):
+    q = torch.ones(1, 2, 130, 128, device="cuda").half()
+    k = torch.ones(1, 1, 130, 128, device="cuda").half()
+    v = torch.randn(1, 1, 130, 128, device="cuda").half()
+    k[0, 0, 64] = float("inf")
+    out = prefill_attention(q, k, v)
+    assert bool(torch.isfinite(out[:, :, :64]).all()) and bool(torch.isnan(out[:, :, 64:]).all())
