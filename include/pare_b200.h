@@ -174,6 +174,28 @@ int pare_kivi_append(const void* k_src, const void* v_src, int src_dtype,
                      uint8_t* v_codes, float* v_scale, float* v_zero,
                      int B, int H, int D, int bits, int group, int v_group, int cap, void* stream);
 
+/* The same with separate strides for keys and values (a prompt's k and v are often views of one fused projection). */
+int pare_kivi_append_kv(const void* k_src, const void* v_src, int src_dtype,
+                        int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_t,
+                        int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_t,
+                        int n_tokens, int t0,
+                        uint8_t* k_codes, float* k_scale, float* k_zero,
+                        uint8_t* v_codes, float* v_scale, float* v_zero,
+                        int B, int H, int D, int bits, int group, int v_group, int cap, void* stream);
+
+/* Everything update() returns, in one launch: the dense reconstruction of compressed tokens 0..n_comp-1, then the
+ * n_res tokens of the full-precision window, then n_new tokens of new_k / new_v, which are stored at the end of the
+ * window on the way (window rows n_res .. n_res+n_new-1).  All of one dtype; 16-byte aligned rows; D = 128 and 2- or
+ * 4-bit codes (PARE_ERR_UNSUPPORTED otherwise: copy the window and use pare_kivi_dequant).  pare/kv_cache.py:244-252. */
+int pare_kivi_dense(const uint8_t* k_codes, const float* k_scale, const float* k_zero,
+                    const uint8_t* v_codes, const float* v_scale, const float* v_zero,
+                    int B, int H, int D, int bits, int group, int v_group, int cap, int n_comp,
+                    void* out_k, void* out_v, int dtype, int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_t,
+                    void* res_k, void* res_v, int64_t res_stride_b, int64_t res_stride_h, int64_t res_stride_t, int n_res,
+                    const void* new_k, const void* new_v,
+                    int64_t new_k_stride_b, int64_t new_k_stride_h, int64_t new_k_stride_t,
+                    int64_t new_v_stride_b, int64_t new_v_stride_h, int64_t new_v_stride_t, int n_new, void* stream);
+
 /* Dense reconstruction code*scale+zero of compressed tokens 0..n_comp-1 into
  * out_k / out_v [B][H][>=n_comp][D] (out_dtype F16/BF16/F32, element strides given).
  * pare/kv_cache.py:315-325 (the part of update()'s return value that comes from the

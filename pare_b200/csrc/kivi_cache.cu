@@ -18,6 +18,8 @@
 //   code  = rint(min(max((x - min) / scale, 0), qmax))   true division, clamp, then half-to-even
 //   x^    = code * scale + min                     separate multiply and add (no FMA contraction)
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace pare {
@@ -44,31 +46,51 @@ __device__ __forceinline__ uint8_t affine_code(float x, float lo, float scale, f
   return (uint8_t)rintf(q);
 }
 
-// The same code without a division per element.  The quotient is approximated by a product with the correctly
-// rounded reciprocal (error below 2 units in the last place of a number below 16, i.e. < 4e-6) and rounded to the
-// nearest integer by adding 1.5 * 2^23 (round-to-nearest-even, like rintf; the integer then sits in the low mantissa
-// bits).  Only an approximation within 1e-4 of a rounding boundary could round differently from the exact quotient:
-// those elements (about one in ten thousand) take the division.  x >= lo by construction, so only the upper clamp is
-// needed.  Bit-identical to affine_code.
-__device__ __forceinline__ uint32_t affine_code_fast(float x, float lo, float inv, const float* scale_ptr, float qmax) {
-  const float q = fminf(__fmul_rn(__fsub_rn(x, lo), inv), qmax);
-  const float r = __fadd_rn(q, 12582912.f);
-  const float frac = __fsub_rn(__fsub_rn(r, 12582912.f), q);
-  if (fabsf(frac) > 0.4999f) return affine_code(x, lo, *scale_ptr, qmax);
-  return __float_as_uint(r) & 0xffu;
+// Eight such codes without a division per element, packed code k at bit k * BITS.  A quotient is approximated by a
+// product with the correctly rounded reciprocal (error below 2 units in the last place of a number below 16, i.e. < 4e-6)
+// and rounded to the nearest integer by adding 1.5 * 2^23 (round-to-nearest-even, like rintf; the integer then sits in the
+// low mantissa bits, and the eight shifted words are added up, the exponent bits taken off once).  Only an approximation
+// within 1e-4 of a rounding boundary could round differently from the exact quotient: one branch per eight elements
+// sends those (about one set in six hundred) through the division.  x >= lo by construction, so only the upper clamp
+// is needed.  Bit-identical to affine_code.
+template <int BITS>
+__device__ __forceinline__ uint32_t affine_codes8(const float (&x)[8], const float (&lo)[8], const float (&inv)[8], const float (&scale)[8]) {
+  constexpr float qmax = (float)((1 << BITS) - 1);
+  constexpr uint32_t kMagic = 0x4B400000u;
+  uint32_t w = 0, fix = 0;
+  float worst = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float q = fminf(__fmul_rn(__fsub_rn(x[k], lo[k]), inv[k]), qmax);
+    const float r = __fadd_rn(q, 12582912.f);
+    worst = fmaxf(worst, fabsf(__fsub_rn(__fsub_rn(r, 12582912.f), q)));
+    w += __float_as_uint(r) << (k * BITS);
+    fix += kMagic << (k * BITS);
+  }
+  w -= fix;
+  if (worst > 0.4999f) {
+    w = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) w |= (uint32_t)affine_code(x[k], lo[k], scale[k], qmax) << (k * BITS);
+  }
+  return w;
 }
+
+struct SrcStrides {
+  int64_t b, h, t;
+};
 
 // One CTA per (token group, head, batch); blockDim.x == D.
 template <typename T>
-__global__ void kivi_append_kernel(const void* k_src, const void* v_src, int64_t sb, int64_t sh, int64_t st, int t0,
-                                   CachePtrs c) {
+__global__ void kivi_append_kernel(const void* k_src, const void* v_src, SrcStrides ks, SrcStrides vs, int t0, CachePtrs c) {
   extern __shared__ unsigned char smem[];
   const int G = c.group, D = c.D, bits = c.bits;
   const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int d = threadIdx.x, warp = d >> 5, lane = d & 31, nwarps = D >> 5;
   const float qmax = (float)((1 << bits) - 1);
   const int tok0 = t0 + g * G;                      // first destination token of this group
-  const int64_t src0 = (int64_t)b * sb + (int64_t)h * sh + (int64_t)g * G * st;
+  const int64_t k0 = (int64_t)b * ks.b + (int64_t)h * ks.h + (int64_t)g * G * ks.t;
+  const int64_t v0 = (int64_t)b * vs.b + (int64_t)h * vs.h + (int64_t)g * G * vs.t;
   const size_t bh = (size_t)b * c.H + h;
 
   uint8_t* codes = smem;                                                   // [G][D]
@@ -80,7 +102,7 @@ __global__ void kivi_append_kernel(const void* k_src, const void* v_src, int64_t
   {
     float lo = INFINITY, hi = -INFINITY;
     for (int t = 0; t < G; ++t) {
-      const float x = load_as_float<T>(k_src, src0 + (int64_t)t * st + d);
+      const float x = load_as_float<T>(k_src, k0 + (int64_t)t * ks.t + d);
       lo = fminf(lo, x);
       hi = fmaxf(hi, x);
     }
@@ -89,7 +111,7 @@ __global__ void kivi_append_kernel(const void* k_src, const void* v_src, int64_t
     c.k_scale[mi] = scale;
     c.k_zero[mi] = lo;
     for (int t = 0; t < G; ++t) {
-      const float x = load_as_float<T>(k_src, src0 + (int64_t)t * st + d);
+      const float x = load_as_float<T>(k_src, k0 + (int64_t)t * ks.t + d);
       codes[t * D + d] = affine_code(x, lo, scale, qmax);
     }
   }
@@ -112,7 +134,7 @@ __global__ void kivi_append_kernel(const void* k_src, const void* v_src, int64_t
     for (int vg = 0; vg < VG; ++vg) {
       float lo = INFINITY, hi = -INFINITY;
       for (int cc = vg * c.v_group + lane; cc < (vg + 1) * c.v_group; cc += 32) {
-        const float x = load_as_float<T>(v_src, src0 + (int64_t)t * st + cc);
+        const float x = load_as_float<T>(v_src, v0 + (int64_t)t * vs.t + cc);
         lo = fminf(lo, x);
         hi = fmaxf(hi, x);
       }
@@ -135,7 +157,7 @@ __global__ void kivi_append_kernel(const void* k_src, const void* v_src, int64_t
       uint32_t v = 0;
       for (int e = 0; e < per_byte; ++e) {
         const int t = tb + e;
-        const float x = load_as_float<T>(v_src, src0 + (int64_t)t * st + d);
+        const float x = load_as_float<T>(v_src, v0 + (int64_t)t * vs.t + d);
         v |= (uint32_t)affine_code(x, v_lo[t * VG + d / c.v_group], v_sc[t * VG + d / c.v_group], qmax) << (e * bits);
       }
       const int tok = tok0 + tb;
@@ -149,37 +171,43 @@ __global__ void kivi_append_kernel(const void* k_src, const void* v_src, int64_t
 // to 64 tokens, 16-byte aligned source rows): one CTA of 128 threads per (token group, head, batch).  The group's keys
 // and values (G x 256 bytes each) come in with 16-byte loads into shared memory and every later pass reads them from
 // there; the codes leave as 16-byte vectors -- a token's key codes in runs of 16 bytes, a channel's value codes of
-// the group as one piece of its row.  Same arithmetic, in the same order, as the element-wise kernel above.
-template <typename T, int BITS, int VG>
-__global__ void __launch_bounds__(128) kivi_append128_kernel(const void* k_src, const void* v_src, int64_t sb, int64_t sh, int64_t st,
-                                                              int t0, CachePtrs c) {
+// the group in pieces of its row.  Same arithmetic, in the same order, as the element-wise kernel above.
+// The group size is a template parameter: with run-time trip counts the shared-memory reads of the statistics and of the
+// value codes were one round trip each (128 threads, 0.26 of the HBM rate); unrolled they overlap.
+__host__ __device__ constexpr int key_pair_slot(int c) {   // (minimum, 1 / scale) of channel c, 8 bytes each: a quarter warp's eight readers (below) hit eight bank groups
+  return 2 * ((c >> 5) * 24 + ((c >> 3) & 3) * 4 + 2 * (((c >> 3) & 3) >> 1) + ((c >> 5) & 1) + ((c & 7) >> 1)) + (c & 1);
+}
+constexpr int kKeyPairs = 192;         // slots, some unused
+
+template <typename T, int BITS, int VG, int G>
+__global__ void __launch_bounds__(128) kivi_append128_kernel(const void* k_src, const void* v_src, SrcStrides ks, SrcStrides vs, int t0,
+                                                              CachePtrs c) {
   constexpr int D = 128;
   extern __shared__ __align__(16) unsigned char sm[];
-  const int G = c.group;
   T* kt = reinterpret_cast<T*>(sm);                         // [G][D]
   T* vt = kt + G * D;                                       // [G][D]
-  float* ks_s = reinterpret_cast<float*>(vt + G * D);       // [D] scale, channel order
-  float* kl_s = ks_s + D;                                   // [D] group minimum
-  float* ki_s = kl_s + D;                                   // [D] 1 / scale
-  float* vs_s = ki_s + D;                                   // [G][VG]
-  float* vl_s = vs_s + G * VG;                              // [G][VG]
-  float* vi_s = vl_s + G * VG;                              // [G][VG] 1 / scale
+  float2* kp_s = reinterpret_cast<float2*>(vt + G * D);     // [key_pair_slot(channel)] (group minimum, 1 / scale)
+  float2* vp_s = kp_s + kKeyPairs;                          // [G][VG] (minimum, 1 / scale)
+  float* ks_s = reinterpret_cast<float*>(vp_s + G * VG);    // [D] scale
+  float* vs_s = ks_s + D;                                   // [G][VG] scale
   const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float qmax = (float)((1 << BITS) - 1);
   const int tok0 = t0 + g * G;
   const size_t bh = (size_t)b * c.H + h;
-  const T* kg = reinterpret_cast<const T*>(k_src) + (int64_t)b * sb + (int64_t)h * sh + (int64_t)g * G * st;
-  const T* vg_ = reinterpret_cast<const T*>(v_src) + (int64_t)b * sb + (int64_t)h * sh + (int64_t)g * G * st;
-  for (int i = tid; i < G * 16; i += 128) {
-    const int t = i >> 4, part = i & 15;
-    reinterpret_cast<uint4*>(kt)[i] = __ldg(reinterpret_cast<const uint4*>(kg + (int64_t)t * st) + part);
-    reinterpret_cast<uint4*>(vt)[i] = __ldg(reinterpret_cast<const uint4*>(vg_ + (int64_t)t * st) + part);
+  const T* kg = reinterpret_cast<const T*>(k_src) + (int64_t)b * ks.b + (int64_t)h * ks.h + (int64_t)g * G * ks.t;
+  const T* vg_ = reinterpret_cast<const T*>(v_src) + (int64_t)b * vs.b + (int64_t)h * vs.h + (int64_t)g * G * vs.t;
+#pragma unroll
+  for (int i0 = 0; i0 < G * 16; i0 += 128) {
+    const int i = i0 + tid, t = i >> 4, part = i & 15;
+    reinterpret_cast<uint4*>(kt)[i] = __ldg(reinterpret_cast<const uint4*>(kg + (int64_t)t * ks.t) + part);
+    reinterpret_cast<uint4*>(vt)[i] = __ldg(reinterpret_cast<const uint4*>(vg_ + (int64_t)t * vs.t) + part);
   }
   __syncthreads();
   // ---- keys: per channel over the G tokens of the group ----
   {
     const int d = tid;
     float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
     for (int t = 0; t < G; ++t) {
       const float x = to_float<T>(kt[t * D + d]);
       lo = fminf(lo, x);
@@ -190,10 +218,10 @@ __global__ void __launch_bounds__(128) kivi_append128_kernel(const void* k_src, 
     c.k_scale[mi] = scale;
     c.k_zero[mi] = lo;
     ks_s[d] = scale;
-    kl_s[d] = lo;
-    ki_s[d] = __frcp_rn(scale);
+    kp_s[key_pair_slot(d)] = make_float2(lo, __frcp_rn(scale));
   }
   // ---- values: per token over each group of D / VG channels (a warp per token, a lane per four channels) ----
+#pragma unroll
   for (int t = warp; t < G; t += 4) {
     const uint2 raw = *reinterpret_cast<const uint2*>(vt + t * D + lane * 4);
     const T* e = reinterpret_cast<const T*>(&raw);
@@ -208,58 +236,95 @@ __global__ void __launch_bounds__(128) kivi_append128_kernel(const void* k_src, 
     if ((lane & (kLanes - 1)) == 0) {
       const float scale = fmaxf(__fdiv_rn(__fsub_rn(hi, lo), qmax), 1e-8f);
       vs_s[t * VG + lane / kLanes] = scale;
-      vl_s[t * VG + lane / kLanes] = lo;
-      vi_s[t * VG + lane / kLanes] = __frcp_rn(scale);
+      vp_s[t * VG + lane / kLanes] = make_float2(lo, __frcp_rn(scale));
     }
   }
   __syncthreads();
   for (int i = tid; i < G * VG; i += 128) {                 // the group's value scales / zeros: contiguous in the cache
     c.v_scale[(bh * c.cap + tok0) * VG + i] = vs_s[i];
-    c.v_zero[(bh * c.cap + tok0) * VG + i] = vl_s[i];
+    c.v_zero[(bh * c.cap + tok0) * VG + i] = vp_s[i].x;
   }
   // ---- key codes: 16 bytes (32 or 64 channels) of one token per step ----
   {
     constexpr int CPI = 128 / BITS;                         // channels per 16 bytes of codes
     constexpr int IPT = D / CPI;                            // such pieces per token
+    constexpr int CH = CPI / 8;                             // 8-channel chunks per piece
     uint8_t* dst = c.k_codes + (bh * c.cap + tok0) * (size_t)(D * BITS / 8);
-    for (int i = tid; i < G * IPT; i += 128) {
-      const int t = i / IPT, c0 = (i % IPT) * CPI;
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-      for (int j = 0; j < CPI; j += 8) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(kt + t * D + c0 + j);
+    for (int i0 = 0; i0 < G * IPT; i0 += 128) {
+      const int i = i0 + tid;
+      if (G * IPT % 128 != 0 && i >= G * IPT) break;
+      const int t = i / IPT, q = i % IPT;
+      // the pieces of a quarter warp start at different chunks, so that its 16-byte reads fall in different banks
+      const int rot = BITS == 4 ? ((q >> 1) + 2 * (t & 1)) & 3 : 0;
+      uint32_t cw[CH];
+#pragma unroll
+      for (int jj = 0; jj < CH; ++jj) {
+        const int c0 = q * CPI + ((jj + rot) & (CH - 1)) * 8;
+        const uint4 raw = *reinterpret_cast<const uint4*>(kt + t * D + c0);
         const T* e = reinterpret_cast<const T*>(&raw);
-        const float4 l0 = *reinterpret_cast<const float4*>(kl_s + c0 + j), l1 = *reinterpret_cast<const float4*>(kl_s + c0 + j + 4);
-        const float4 i0 = *reinterpret_cast<const float4*>(ki_s + c0 + j), i1 = *reinterpret_cast<const float4*>(ki_s + c0 + j + 4);
-        const float lo8[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-        const float in8[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
+        float x[8], lo[8], in[8], sc[8];
+        const float4* pr = reinterpret_cast<const float4*>(kp_s + key_pair_slot(c0));
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t code = affine_code_fast(to_float<T>(e[k]), lo8[k], in8[k], ks_s + c0 + j + k, qmax);
-          w[((j + k) * BITS) >> 5] |= code << (((j + k) * BITS) & 31);
+        for (int k = 0; k < 8; k += 2) {
+          const float4 pv = pr[k >> 1];
+          lo[k] = pv.x; in[k] = pv.y; lo[k + 1] = pv.z; in[k + 1] = pv.w;
         }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = to_float<T>(e[k]), sc[k] = ks_s[c0 + k];
+        cw[jj] = affine_codes8<BITS>(x, lo, in, sc);
+      }
+      uint32_t w[4];
+      if constexpr (BITS == 4) {   // undo the rotation: chunk j was done at place (j - rot) mod 4
+        const bool r1 = rot & 1, r2 = rot & 2;
+        uint32_t m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m[j] = r1 ? cw[(j + 3) & 3] : cw[j];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = r2 ? m[(j + 2) & 3] : m[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = (cw[2 * j] & 0xffffu) | (cw[2 * j + 1] << 16);
       }
       *reinterpret_cast<uint4*>(dst + (size_t)i * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
-  // ---- value codes: thread d packs the group's G tokens of channel d into its row of the 128-token block ----
+  // ---- value codes: a thread packs half of the group's tokens of two neighbouring channels into their rows ----
   {
-    const int d = tid, gi = VG == 1 ? 0 : (d >> 5);
-    constexpr int TPW = 32 / BITS;                          // tokens per 32-bit word
-    uint8_t* row = c.v_codes + ((bh * (c.cap / 128) + tok0 / 128) * D + d) * (size_t)(128 * BITS / 8) + (tok0 % 128) * BITS / 8;
-    const int words = G / TPW;
-    for (int w0 = 0; w0 < words; w0 += 4) {
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
-      const int nw = min(4, words - w0);
-      for (int wi = 0; wi < nw; ++wi)
+    const int d = (tid & 63) * 2, gi = VG == 1 ? 0 : (d >> 5);
+    constexpr int HT = G / 2;                               // tokens per thread
+    const int th = (tid >> 6) * HT;
+    uint32_t w[2][HT / 8];
 #pragma unroll
-        for (int k = 0; k < TPW; ++k) {
-          const int t = (w0 + wi) * TPW + k;
-          w[wi] |= affine_code_fast(to_float<T>(vt[t * D + d]), vl_s[t * VG + gi], vi_s[t * VG + gi], vs_s + t * VG + gi, qmax) << (k * BITS);
-        }
-      if (nw == 4) *reinterpret_cast<uint4*>(row + w0 * 4) = make_uint4(w[0], w[1], w[2], w[3]);
-      else if (nw == 2) *reinterpret_cast<uint2*>(row + w0 * 4) = make_uint2(w[0], w[1]);
-      else for (int wi = 0; wi < nw; ++wi) *reinterpret_cast<uint32_t*>(row + (w0 + wi) * 4) = w[wi];
+    for (int t8 = 0; t8 < HT; t8 += 8) {
+      float x0[8], x1[8], lo[8], in[8], sc[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int t = th + t8 + k;
+        const uint32_t raw = *reinterpret_cast<const uint32_t*>(vt + t * D + d);
+        const T* e = reinterpret_cast<const T*>(&raw);
+        x0[k] = to_float<T>(e[0]);
+        x1[k] = to_float<T>(e[1]);
+        const float2 pv = vp_s[t * VG + gi];
+        lo[k] = pv.x; in[k] = pv.y;
+        sc[k] = vs_s[t * VG + gi];
+      }
+      w[0][t8 / 8] = affine_codes8<BITS>(x0, lo, in, sc);
+      w[1][t8 / 8] = affine_codes8<BITS>(x1, lo, in, sc);
+    }
+    uint8_t* row = c.v_codes + ((bh * (c.cap / 128) + tok0 / 128) * D + d) * (size_t)(128 * BITS / 8) + (tok0 % 128 + th) * BITS / 8;
+#pragma unroll
+    for (int e = 0; e < 2; ++e, row += 128 * BITS / 8) {
+      constexpr int NB = HT * BITS / 8;                     // bytes: 2, 4, 8 or 16
+      if constexpr (BITS == 4) {
+        if constexpr (NB == 16) *reinterpret_cast<uint4*>(row) = make_uint4(w[e][0], w[e][1], w[e][2], w[e][3]);
+        else if constexpr (NB == 8) *reinterpret_cast<uint2*>(row) = make_uint2(w[e][0], w[e][1]);
+        else *reinterpret_cast<uint32_t*>(row) = w[e][0];
+      } else {
+        if constexpr (NB == 8) *reinterpret_cast<uint2*>(row) = make_uint2((w[e][0] & 0xffffu) | (w[e][1] << 16), (w[e][2] & 0xffffu) | (w[e][3] << 16));
+        else if constexpr (NB == 4) *reinterpret_cast<uint32_t*>(row) = (w[e][0] & 0xffffu) | (w[e][1] << 16);
+        else *reinterpret_cast<uint16_t*>(row) = (uint16_t)w[e][0];
+      }
     }
   }
 }
@@ -306,36 +371,93 @@ __device__ __forceinline__ void store8(T* dst, const float (&v)[8]) {
   }
 }
 
+// (2^23 + q 2^p) - 2^23 for two codes at once (exact), then times scale plus zero, each rounded separately.  Product and
+// sum are scalar on purpose: the compiler contracts a packed multiply and add into one fused operation.
+__device__ __forceinline__ void affine_pair(float& a, float& b, float s0, float s1, float z0, float z1) {
+  asm("{\n\t.reg .b64 x, m;\n\t"
+      "mov.b64 x, {%0, %1};\n\t"
+      "mov.b64 m, {%2, %2};\n\t"
+      "add.rn.f32x2 x, x, m;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(a), "+f"(b)
+      : "f"(-8388608.f));
+  a = __fadd_rn(__fmul_rn(a, s0), z0);
+  b = __fadd_rn(__fmul_rn(b, s1), z1);
+}
+
+// What update() returns beside the reconstructed tokens: the full-precision window, and tokens that are only now arriving
+struct WindowArgs {
+  void* res_k;              // [B][H][..][128] window, n_old tokens of it in use
+  void* res_v;
+  const void* new_k;        // n_new tokens that are copied into the window and the result on the way
+  const void* new_v;
+  SrcStrides r, nk, nv;
+  int n_old, n_new;
+};
+
 // Vectorised dequantize for the attention geometry (D == 128, 2- or 4-bit codes, 16-byte aligned output rows): one
 // CTA of 256 threads per (128-token block, head, batch).  The block's codes and metadata (about 21 KB) come in with
-// 16-byte loads into shared memory; a thread then produces eight consecutive channels of one token at a time --
-// the key codes of such a run are one 32-bit (16-bit) word, the value codes one nibble from each of eight channel
-// rows -- and stores them as one 16-byte vector, a token's 256 output bytes contiguous across 16 threads.
+// 16-byte loads into shared memory; a thread then produces EIGHT TOKENS of eight consecutive channels: one code word per
+// token (keys) or channel (values) and the keys' scales and zeros in registers for all eight, sixteen 16-byte stores,
+// a token's 256 output bytes contiguous across 16 threads.  (One token at a time took a shared-memory byte read per
+// value code and an integer-to-float conversion per element: 0.44 - 0.51 of the HBM rate.)  A code left in place at bit p
+// of a float's mantissa under the exponent of 2^23 is 2^23 + code * 2^p; taking 2^23 off is exact, and the 2^p goes into
+// the scale, which a power of two leaves exact: the product rounds like code * scale.
+// CTAs beyond the compressed blocks copy 128 tokens of the window each (WindowArgs).
 template <typename T, int BITS, int VG>
-__global__ void __launch_bounds__(256) kivi_dequant128_kernel(CachePtrs c, int n_comp, void* out_k, void* out_v, int64_t ob, int64_t oh,
-                                                               int64_t ot) {
-  constexpr int D = 128, KROW = D * BITS / 8, VROW = 128 * BITS / 8, VPITCH = VROW + 4;   // value rows padded: conflict-free column reads
+__global__ void __launch_bounds__(256) kivi_dequant128_kernel(CachePtrs c, int n_comp, int n_blocks, void* out_k, void* out_v, int64_t ob,
+                                                               int64_t oh, int64_t ot, const WindowArgs win) {
+  constexpr int D = 128, KROW = D * BITS / 8, VROW = 128 * BITS / 8;
   extern __shared__ __align__(16) unsigned char sm[];
   const int G = c.group, ngr = 128 / G;
-  unsigned char* kc = sm;                                              // [128][KROW]
-  unsigned char* vc = kc + 128 * KROW;                                 // [D][VPITCH]
-  float* ks = reinterpret_cast<float*>(vc + D * VPITCH);               // [ngr][D] in kmeta_pos order
+  const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
+  T* okp = reinterpret_cast<T*>(out_k) + (int64_t)b * ob + (int64_t)h * oh;
+  T* ovp = reinterpret_cast<T*>(out_v) + (int64_t)b * ob + (int64_t)h * oh;
+  if (blk >= n_blocks) {
+    constexpr int kVec = 16 / (int)sizeof(T), kPer = D / kVec;   // 16-byte pieces per row
+    const int w0 = (blk - n_blocks) * 128, n = min(128, win.n_old + win.n_new - w0);
+    T* rk = reinterpret_cast<T*>(win.res_k) + (int64_t)b * win.r.b + (int64_t)h * win.r.h;
+    T* rv = reinterpret_cast<T*>(win.res_v) + (int64_t)b * win.r.b + (int64_t)h * win.r.h;
+    const T* nk = reinterpret_cast<const T*>(win.new_k) + (int64_t)b * win.nk.b + (int64_t)h * win.nk.h;
+    const T* nv = reinterpret_cast<const T*>(win.new_v) + (int64_t)b * win.nv.b + (int64_t)h * win.nv.h;
+    for (int i = tid; i < n * kPer; i += 256) {
+      const int t = w0 + i / kPer, at = (i % kPer) * kVec;
+      const bool fresh = t >= win.n_old;
+      const uint4 kq = *reinterpret_cast<const uint4*>(fresh ? nk + (int64_t)(t - win.n_old) * win.nk.t + at : rk + (int64_t)t * win.r.t + at);
+      const uint4 vq = *reinterpret_cast<const uint4*>(fresh ? nv + (int64_t)(t - win.n_old) * win.nv.t + at : rv + (int64_t)t * win.r.t + at);
+      *reinterpret_cast<uint4*>(okp + (int64_t)(n_comp + t) * ot + at) = kq;
+      *reinterpret_cast<uint4*>(ovp + (int64_t)(n_comp + t) * ot + at) = vq;
+      if (fresh) {
+        *reinterpret_cast<uint4*>(rk + (int64_t)t * win.r.t + at) = kq;
+        *reinterpret_cast<uint4*>(rv + (int64_t)t * win.r.t + at) = vq;
+      }
+    }
+    return;
+  }
+  // rows of eight tokens (keys) / channels (values) are skewed so that a warp's word reads fall in different banks
+  constexpr int KSKEW = KROW, VSKEW = 8;
+  unsigned char* kc = sm;                                              // [128][KROW], + KSKEW every 8 rows
+  unsigned char* vc = kc + 128 * KROW + 16 * KSKEW;                    // [D][VROW], + VSKEW every 8 rows
+  float* ks = reinterpret_cast<float*>(vc + D * VROW + 16 * VSKEW);    // [ngr][D] in kmeta_pos order
   float* kz = ks + ngr * D;
   float* vs = kz + ngr * D;                                            // [128][VG]
   float* vz = vs + 128 * VG;
-  const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
   const size_t bh = (size_t)b * c.H + h;
   const int t0 = blk * 128, valid = min(128, n_comp - t0);             // a multiple of G
   const int vgroups = valid / G;
   {
     const uint4* src = reinterpret_cast<const uint4*>(c.k_codes + (bh * c.cap + t0) * (size_t)KROW);
-    for (int i = tid; i < valid * KROW / 16; i += 256) reinterpret_cast<uint4*>(kc)[i] = __ldg(src + i);
+    for (int i = tid; i < valid * KROW / 16; i += 256) {
+      const int row = i / (KROW / 16);
+      *reinterpret_cast<uint4*>(kc + i * 16 + (row >> 3) * KSKEW) = __ldg(src + i);
+    }
     const uint4* vsrc = reinterpret_cast<const uint4*>(c.v_codes + (bh * (c.cap / 128) + blk) * (size_t)(D * VROW));
     for (int i = tid; i < D * VROW / 16; i += 256) {
       const uint4 v = __ldg(vsrc + i);
-      const int row = i / (VROW / 16), part = i % (VROW / 16);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(vc + row * VPITCH + part * 16);   // rows are only 4-byte aligned
-      dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
+      const int row = i / (VROW / 16);
+      uint2* dst = reinterpret_cast<uint2*>(vc + i * 16 + (row >> 3) * VSKEW);   // 8-byte aligned
+      dst[0] = make_uint2(v.x, v.y);
+      dst[1] = make_uint2(v.z, v.w);
     }
     const size_t grow = (bh * (c.cap / G) + t0 / G) * D;
     for (int i = tid; i < vgroups * D / 4; i += 256) {
@@ -349,34 +471,57 @@ __global__ void __launch_bounds__(256) kivi_dequant128_kernel(CachePtrs c, int n
     }
   }
   __syncthreads();
-  T* okp = reinterpret_cast<T*>(out_k) + (int64_t)b * ob + (int64_t)h * oh;
-  T* ovp = reinterpret_cast<T*>(out_v) + (int64_t)b * ob + (int64_t)h * oh;
-  constexpr uint32_t MASK = (1u << BITS) - 1u;
-  for (int item = tid; item < valid * 16; item += 256) {   // (token, run of eight channels)
-    const int t = item >> 4, r = item & 15, c8 = r * 8;
-    // ---- keys: the run's codes are BITS bytes of the token's row ----
-    uint32_t kw;
-    if constexpr (BITS == 4) kw = *reinterpret_cast<const uint32_t*>(kc + t * KROW + r * 4);
-    else kw = *reinterpret_cast<const uint16_t*>(kc + t * KROW + r * 2);
-    const int mp = (t / G) * D + kmeta_pos(c8, D);          // the eight channels of a run are adjacent in the stored order
+  const int tg = tid >> 4, r = tid & 15, c8 = r * 8, tl = tg * 8;      // tokens tl .. tl + 7 (one group: groups are multiples of 16)
+  if (tl >= valid) return;
+  constexpr uint32_t kMagic = 0x4B000000u;
+  // code j of a word as 2^23 + code * 2^(shift_of(j)); 4-bit words are read in two halves
+  auto place = [](uint32_t w, int j) -> float {
+    if constexpr (BITS == 4) return __uint_as_float(and_or(j < 4 ? w : w >> 16, 0xFu << (4 * (j & 3)), kMagic));
+    else return __uint_as_float(and_or(w, 0x3u << (2 * j), kMagic));
+  };
+  auto unit = [](int j) -> float {   // 2^-shift_of(j)
+    return __int_as_float((127 - (BITS == 4 ? 4 * (j & 3) : 2 * j)) << 23);
+  };
+  {  // ---- keys ----
+    const int mp = (tl / G) * D + kmeta_pos(c8, D);          // the eight channels of a run are adjacent in the stored order
     const float4 s0 = *reinterpret_cast<const float4*>(ks + mp), s1 = *reinterpret_cast<const float4*>(ks + mp + 4);
     const float4 z0 = *reinterpret_cast<const float4*>(kz + mp), z1 = *reinterpret_cast<const float4*>(kz + mp + 4);
-    const float sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+    float sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
     const float zv[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
-    float kv[8], vv[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) kv[j] = __fadd_rn(__fmul_rn((float)((kw >> (j * BITS)) & MASK), sv[j]), zv[j]);
-    store8<T>(okp + (int64_t)(t0 + t) * ot + c8, kv);
-    // ---- values: one code from each of the run's eight channel rows ----
+    for (int j = 0; j < 8; ++j) sv[j] *= unit(j);
+    T* dst = okp + (int64_t)(t0 + tl) * ot + c8;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const unsigned char* at = kc + (tl + t) * KROW + tg * KSKEW + r * BITS;
+      const uint32_t w = BITS == 4 ? *reinterpret_cast<const uint32_t*>(at) : *reinterpret_cast<const uint16_t*>(at);
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = place(w, j);
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) affine_pair(v[j], v[j + 1], sv[j], sv[j + 1], zv[j], zv[j + 1]);
+      store8<T>(dst + (int64_t)t * ot, v);
+    }
+  }
+  {  // ---- values: word j holds the eight tokens of channel c8 + j ----
     const int vgi = VG == 1 ? 0 : (c8 >> 5);
-    const float vsc = vs[t * VG + vgi], vzr = vz[t * VG + vgi];
-    const int byte = (t * BITS) >> 3, sh = (t * BITS) & 7;
+    uint32_t w[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const uint32_t code = (vc[(c8 + j) * VPITCH + byte] >> sh) & MASK;
-      vv[j] = __fadd_rn(__fmul_rn((float)code, vsc), vzr);
+      const unsigned char* at = vc + (c8 + j) * VROW + r * VSKEW + tg * BITS;
+      w[j] = BITS == 4 ? *reinterpret_cast<const uint32_t*>(at) : *reinterpret_cast<const uint16_t*>(at);
     }
-    store8<T>(ovp + (int64_t)(t0 + t) * ot + c8, vv);
+    T* dst = ovp + (int64_t)(t0 + tl) * ot + c8;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const float s = vs[(tl + t) * VG + vgi] * unit(t), z = vz[(tl + t) * VG + vgi];
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = place(w[j], t);
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) affine_pair(v[j], v[j + 1], s, s, z, z);
+      store8<T>(dst + (int64_t)t * ot, v);
+    }
   }
 }
 
@@ -398,10 +543,10 @@ using pare::CachePtrs;
 
 extern "C" {
 
-int pare_kivi_append(const void* k_src, const void* v_src, int src_dtype, int64_t stride_b, int64_t stride_h,
-                     int64_t stride_t, int n_tokens, int t0, uint8_t* k_codes, float* k_scale, float* k_zero,
-                     uint8_t* v_codes, float* v_scale, float* v_zero, int B, int H, int D, int bits, int group, int v_group,
-                     int cap, void* stream) {
+int pare_kivi_append_kv(const void* k_src, const void* v_src, int src_dtype, int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_t,
+                        int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_t, int n_tokens, int t0, uint8_t* k_codes,
+                        float* k_scale, float* k_zero, uint8_t* v_codes, float* v_scale, float* v_zero, int B, int H, int D, int bits,
+                        int group, int v_group, int cap, void* stream) {
   CachePtrs c{k_codes, k_scale, k_zero, v_codes, v_scale, v_zero, B, H, D, bits, group, cap, v_group > 0 ? v_group : D};
   const int rc = pare::check_cache(c);
   if (rc != PARE_OK) return rc;
@@ -409,38 +554,107 @@ int pare_kivi_append(const void* k_src, const void* v_src, int src_dtype, int64_
   PARE_REQUIRE(n_tokens % group == 0 && t0 >= 0 && t0 % group == 0 && t0 + n_tokens <= cap, PARE_ERR_SHAPE);
   const dim3 grid(n_tokens / group, H, B);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const pare::SrcStrides ks{k_stride_b, k_stride_h, k_stride_t}, vst{v_stride_b, v_stride_h, v_stride_t};
   const int vg = D / c.v_group;
-  if (D == 128 && (bits == 2 || bits == 4) && (vg == 1 || vg == 4) && group <= 64 && (src_dtype == PARE_F16 || src_dtype == PARE_BF16) &&
-      pare::aligned16(k_src) && pare::aligned16(v_src) && stride_b % 8 == 0 && stride_h % 8 == 0 && stride_t % 8 == 0 &&
-      pare::aligned16(k_codes) && pare::aligned16(v_codes)) {
-    const size_t smem = (size_t)2 * group * 128 * 2 + 3 * 128 * sizeof(float) + 3 * (size_t)group * vg * sizeof(float);
-#define PARE_AP(T)                                                                                                                   \
-  do {                                                                                                                               \
-    if (bits == 4 && vg == 1) pare::kivi_append128_kernel<T, 4, 1><<<grid, 128, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c); \
-    else if (bits == 4) pare::kivi_append128_kernel<T, 4, 4><<<grid, 128, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c);       \
-    else if (vg == 1) pare::kivi_append128_kernel<T, 2, 1><<<grid, 128, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c);         \
-    else pare::kivi_append128_kernel<T, 2, 4><<<grid, 128, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c);                      \
-  } while (0)
-    if (src_dtype == PARE_F16) PARE_AP(__half);
-    else PARE_AP(__nv_bfloat16);
-#undef PARE_AP
-    return pare::launch_status();
+  bool vec = true;
+  for (int64_t st : {k_stride_b, k_stride_h, k_stride_t, v_stride_b, v_stride_h, v_stride_t}) vec = vec && st % 8 == 0;
+  if (vec && D == 128 && (bits == 2 || bits == 4) && (vg == 1 || vg == 4) && group <= 64 && (src_dtype == PARE_F16 || src_dtype == PARE_BF16) &&
+      pare::aligned16(k_src) && pare::aligned16(v_src) && pare::aligned16(k_codes) && pare::aligned16(v_codes)) {
+    const size_t smem = (size_t)2 * group * 128 * 2 + pare::kKeyPairs * sizeof(float2) + 128 * sizeof(float) + 3 * (size_t)group * vg * sizeof(float);
+    auto launch = [&](auto t_tag, auto bits_tag, auto vg_tag) -> int {
+      using T = decltype(t_tag);
+      constexpr int BITS = decltype(bits_tag)::value, VG = decltype(vg_tag)::value;
+      if (group == 16) pare::kivi_append128_kernel<T, BITS, VG, 16><<<grid, 128, smem, s>>>(k_src, v_src, ks, vst, t0, c);
+      else if (group == 32) pare::kivi_append128_kernel<T, BITS, VG, 32><<<grid, 128, smem, s>>>(k_src, v_src, ks, vst, t0, c);
+      else pare::kivi_append128_kernel<T, BITS, VG, 64><<<grid, 128, smem, s>>>(k_src, v_src, ks, vst, t0, c);
+      return pare::launch_status();
+    };
+    using std::integral_constant;
+    auto pick = [&](auto t_tag) -> int {
+      if (bits == 4) return vg == 1 ? launch(t_tag, integral_constant<int, 4>{}, integral_constant<int, 1>{}) : launch(t_tag, integral_constant<int, 4>{}, integral_constant<int, 4>{});
+      return vg == 1 ? launch(t_tag, integral_constant<int, 2>{}, integral_constant<int, 1>{}) : launch(t_tag, integral_constant<int, 2>{}, integral_constant<int, 4>{});
+    };
+    return src_dtype == PARE_F16 ? pick(__half{}) : pick(__nv_bfloat16{});
   }
   const size_t smem = (size_t)group * D + 2 * group * (D / c.v_group) * sizeof(float);
   switch (src_dtype) {
     case PARE_F16:
-      pare::kivi_append_kernel<__half><<<grid, D, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c);
+      pare::kivi_append_kernel<__half><<<grid, D, smem, s>>>(k_src, v_src, ks, vst, t0, c);
       break;
     case PARE_BF16:
-      pare::kivi_append_kernel<__nv_bfloat16><<<grid, D, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c);
+      pare::kivi_append_kernel<__nv_bfloat16><<<grid, D, smem, s>>>(k_src, v_src, ks, vst, t0, c);
       break;
     case PARE_F32:
-      pare::kivi_append_kernel<float><<<grid, D, smem, s>>>(k_src, v_src, stride_b, stride_h, stride_t, t0, c);
+      pare::kivi_append_kernel<float><<<grid, D, smem, s>>>(k_src, v_src, ks, vst, t0, c);
       break;
     default:
       return PARE_ERR_DTYPE;
   }
   return pare::launch_status();
+}
+
+int pare_kivi_append(const void* k_src, const void* v_src, int src_dtype, int64_t stride_b, int64_t stride_h,
+                     int64_t stride_t, int n_tokens, int t0, uint8_t* k_codes, float* k_scale, float* k_zero,
+                     uint8_t* v_codes, float* v_scale, float* v_zero, int B, int H, int D, int bits, int group, int v_group,
+                     int cap, void* stream) {
+  return pare_kivi_append_kv(k_src, v_src, src_dtype, stride_b, stride_h, stride_t, stride_b, stride_h, stride_t, n_tokens, t0, k_codes,
+                             k_scale, k_zero, v_codes, v_scale, v_zero, B, H, D, bits, group, v_group, cap, stream);
+}
+
+static int dequant128(const CachePtrs& c, int n_comp, void* out_k, void* out_v, int out_dtype, int64_t stride_b, int64_t stride_h,
+                      int64_t stride_t, const pare::WindowArgs& win, void* stream) {
+  const int vg = c.D / c.v_group, bits = c.bits;
+  const size_t esz = out_dtype == PARE_F32 ? 4 : 2;
+  const bool fast = c.D == 128 && (bits == 2 || bits == 4) && (vg == 1 || vg == 4) && pare::aligned16(out_k) && pare::aligned16(out_v) &&
+                    (stride_b * esz) % 16 == 0 && (stride_h * esz) % 16 == 0 && (stride_t * esz) % 16 == 0 &&
+                    pare::aligned16(c.k_codes) && pare::aligned16(c.v_codes) && pare::aligned16(c.k_scale) && pare::aligned16(c.k_zero) &&
+                    pare::aligned16(c.v_scale) && pare::aligned16(c.v_zero);
+  if (!fast) return PARE_ERR_UNSUPPORTED;
+  const int n_blocks = (n_comp + 127) / 128;
+  const dim3 grid(n_blocks + (win.n_old + win.n_new + 127) / 128, c.H, c.B);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const size_t row = 128 * bits / 8;
+  const size_t smem = 128 * row + 16 * row + 128 * row + 16 * 8 + 2 * (size_t)(128 / c.group) * 128 * 4 + 2 * (size_t)128 * vg * 4;
+  auto launch = [&](auto kern) -> int {
+    if (smem > 48 * 1024 && !pare::ensure_smem_attr(reinterpret_cast<const void*>(kern), 64 * 1024)) return PARE_ERR_CUDA;
+    kern<<<grid, 256, smem, s>>>(c, n_comp, n_blocks, out_k, out_v, stride_b, stride_h, stride_t, win);
+    return pare::launch_status();
+  };
+#define PARE_DQ(T)                                                                                        \
+  (bits == 4 ? (vg == 1 ? launch(pare::kivi_dequant128_kernel<T, 4, 1>) : launch(pare::kivi_dequant128_kernel<T, 4, 4>)) \
+             : (vg == 1 ? launch(pare::kivi_dequant128_kernel<T, 2, 1>) : launch(pare::kivi_dequant128_kernel<T, 2, 4>)))
+  switch (out_dtype) {
+    case PARE_F16: return PARE_DQ(__half);
+    case PARE_BF16: return PARE_DQ(__nv_bfloat16);
+    case PARE_F32: return PARE_DQ(float);
+    default: return PARE_ERR_DTYPE;
+  }
+#undef PARE_DQ
+}
+
+int pare_kivi_dense(const uint8_t* k_codes, const float* k_scale, const float* k_zero, const uint8_t* v_codes, const float* v_scale,
+                    const float* v_zero, int B, int H, int D, int bits, int group, int v_group, int cap, int n_comp, void* out_k,
+                    void* out_v, int dtype, int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_t, void* res_k, void* res_v,
+                    int64_t res_stride_b, int64_t res_stride_h, int64_t res_stride_t, int n_res, const void* new_k, const void* new_v,
+                    int64_t new_k_stride_b, int64_t new_k_stride_h, int64_t new_k_stride_t, int64_t new_v_stride_b,
+                    int64_t new_v_stride_h, int64_t new_v_stride_t, int n_new, void* stream) {
+  CachePtrs c{const_cast<uint8_t*>(k_codes), const_cast<float*>(k_scale), const_cast<float*>(k_zero),
+              const_cast<uint8_t*>(v_codes), const_cast<float*>(v_scale), const_cast<float*>(v_zero),
+              B, H, D, bits, group, cap, v_group > 0 ? v_group : D};
+  const int rc = pare::check_cache(c);
+  if (rc != PARE_OK) return rc;
+  PARE_REQUIRE(out_k && out_v && n_comp >= 0 && n_comp <= cap && n_comp % group == 0 && n_res >= 0 && n_new >= 0, PARE_ERR_SHAPE);
+  PARE_REQUIRE(n_res + n_new == 0 || (res_k && res_v), PARE_ERR_SHAPE);
+  PARE_REQUIRE(n_new == 0 || (new_k && new_v), PARE_ERR_SHAPE);
+  if (n_comp + n_res + n_new == 0) return PARE_OK;
+  const size_t esz = dtype == PARE_F32 ? 4 : 2;
+  for (int64_t st : {res_stride_b, res_stride_h, res_stride_t, new_k_stride_b, new_k_stride_h, new_k_stride_t, new_v_stride_b,
+                     new_v_stride_h, new_v_stride_t})
+    PARE_REQUIRE((st * (int64_t)esz) % 16 == 0, PARE_ERR_UNSUPPORTED);
+  PARE_REQUIRE(pare::aligned16(res_k) && pare::aligned16(res_v) && pare::aligned16(new_k) && pare::aligned16(new_v), PARE_ERR_UNSUPPORTED);
+  const pare::WindowArgs win{res_k, res_v, new_k, new_v, {res_stride_b, res_stride_h, res_stride_t},
+                             {new_k_stride_b, new_k_stride_h, new_k_stride_t}, {new_v_stride_b, new_v_stride_h, new_v_stride_t}, n_res, n_new};
+  return dequant128(c, n_comp, out_k, out_v, dtype, out_stride_b, out_stride_h, out_stride_t, win, stream);
 }
 
 int pare_kivi_dequant(const uint8_t* k_codes, const float* k_scale, const float* k_zero, const uint8_t* v_codes,
@@ -454,33 +668,10 @@ int pare_kivi_dequant(const uint8_t* k_codes, const float* k_scale, const float*
   if (rc != PARE_OK) return rc;
   PARE_REQUIRE(out_k && out_v && n_comp >= 0 && n_comp <= cap && n_comp % group == 0, PARE_ERR_SHAPE);
   if (n_comp == 0) return PARE_OK;
+  const int fast = dequant128(c, n_comp, out_k, out_v, out_dtype, stride_b, stride_h, stride_t, pare::WindowArgs{}, stream);
+  if (fast != PARE_ERR_UNSUPPORTED) return fast;
   const dim3 grid((n_comp + 127) / 128, H, B);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int vg = D / c.v_group;
-  const size_t esz = out_dtype == PARE_F32 ? 4 : 2;
-  const bool fast = D == 128 && (bits == 2 || bits == 4) && (vg == 1 || vg == 4) && pare::aligned16(out_k) && pare::aligned16(out_v) &&
-                    (stride_b * esz) % 16 == 0 && (stride_h * esz) % 16 == 0 && (stride_t * esz) % 16 == 0 &&
-                    pare::aligned16(k_codes) && pare::aligned16(v_codes) && pare::aligned16(k_scale) && pare::aligned16(k_zero) &&
-                    pare::aligned16(v_scale) && pare::aligned16(v_zero);
-  if (fast) {
-    const size_t smem = (size_t)128 * (128 * bits / 8) + (size_t)128 * (128 * bits / 8 + 4) + 2 * (size_t)(128 / group) * 128 * 4 +
-                        2 * (size_t)128 * vg * 4;
-    auto launch = [&](auto kern) -> int {
-      if (smem > 48 * 1024 && !pare::ensure_smem_attr(reinterpret_cast<const void*>(kern), 64 * 1024)) return PARE_ERR_CUDA;
-      kern<<<grid, 256, smem, s>>>(c, n_comp, out_k, out_v, stride_b, stride_h, stride_t);
-      return pare::launch_status();
-    };
-#define PARE_DQ(T)                                                                                        \
-  (bits == 4 ? (vg == 1 ? launch(pare::kivi_dequant128_kernel<T, 4, 1>) : launch(pare::kivi_dequant128_kernel<T, 4, 4>)) \
-             : (vg == 1 ? launch(pare::kivi_dequant128_kernel<T, 2, 1>) : launch(pare::kivi_dequant128_kernel<T, 2, 4>)))
-    switch (out_dtype) {
-      case PARE_F16: return PARE_DQ(__half);
-      case PARE_BF16: return PARE_DQ(__nv_bfloat16);
-      case PARE_F32: return PARE_DQ(float);
-      default: return PARE_ERR_DTYPE;
-    }
-#undef PARE_DQ
-  }
   switch (out_dtype) {
     case PARE_F16:
       pare::kivi_dequant_kernel<__half><<<grid, D, 0, s>>>(c, n_comp, out_k, out_v, stride_b, stride_h, stride_t);

@@ -16,6 +16,7 @@ import torch
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libpare_b200.so"
 
 F16, BF16, F32 = 0, 1, 2
+UNSUPPORTED = 5   # PARE_ERR_UNSUPPORTED
 PRODUCER_RMSNORM, PRODUCER_SILU_MUL = 1, 2
 _DTYPE_CODE = {torch.float16: F16, torch.bfloat16: BF16, torch.float32: F32}
 
@@ -40,6 +41,11 @@ SIGNATURES: dict[str, tuple] = {
                                          _i, _i, _i, _i, _vp, _sz, _vp]),
     "pare_kivi_append": (_i, [_vp, _vp, _i, _i64, _i64, _i64, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp,
                               _i, _i, _i, _i, _i, _i, _i, _vp]),
+    "pare_kivi_append_kv": (_i, [_vp, _vp, _i, _i64, _i64, _i64, _i64, _i64, _i64, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp,
+                                 _i, _i, _i, _i, _i, _i, _i, _vp]),
+    "pare_kivi_dense": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
+                             _vp, _vp, _i, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _i,
+                             _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i, _vp]),
     "pare_kivi_dequant": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
                                _vp, _vp, _i, _i64, _i64, _i64, _vp]),
     "pare_kivi_attn_workspace_bytes": (_sz, [_i, _i, _i, _i]),

@@ -261,13 +261,17 @@ class QuantizedKVCache:
             self._stores[layer_idx] = st
         return st
 
-    def _append(self, layer_idx: int, new_k: Tensor, new_v: Tensor, defer_single: bool = False, rope: Tensor | None = None):
+    def _append(self, layer_idx: int, new_k: Tensor, new_v: Tensor, defer_single: bool = False, rope: Tensor | None = None,
+                defer_window: bool = False):
         """Append tokens to the residual window and compress what overflows it.
 
         With ``defer_single`` returns ``(store, deferred)``: when one token arrives and nothing has
         to be compressed, the copy into the window is left to the attention kernel (``deferred``).  ``rope``: rows of
         a :func:`rope_table` for the new tokens; applied to the keys here unless the append is deferred (then the
-        attention kernel does it)."""
+        attention kernel does it).
+
+        With ``defer_window`` returns ``(store, k, v)``: new tokens that end up at the end of the window and that the
+        caller still has to copy there (``None`` where this has been done)."""
         if new_k.shape != new_v.shape or new_k.dim() != 4:
             raise ValueError("new_k / new_v must both be [B, H, new_tokens, D]")
         st = self._store(layer_idx, new_k)
@@ -284,54 +288,91 @@ class QuantizedKVCache:
                     and new_k.stride() == new_v.stride())
         if rope is not None and not deferred:   # the kernel rotates only a key it appends itself
             new_k = apply_rope(new_k, rope)
+        left_k = left_v = None   # with defer_window: what the caller copies into the window
+        # kernels may read the new tokens where they are: same device and dtype as the store, nothing for autograd to see
+        plain = (new_k.device == st.device and new_v.device == st.device and new_v.dtype == st.dtype
+                 and new_k.stride(3) == 1 and new_v.stride(3) == 1
+                 and not (torch.is_grad_enabled() and (new_k.requires_grad or new_v.requires_grad)))
+        from_empty = st.r_len == 0 and plain
         if deferred:
             pass
         elif total <= st.r_cap:
-            st.res_k[:, :, st.r_len:total] = new_k
-            st.res_v[:, :, st.r_len:total] = new_v
+            if defer_window and plain and n_c == 0:
+                left_k, left_v = new_k, new_v
+            else:
+                st.res_k[:, :, st.r_len:total] = new_k
+                st.res_v[:, :, st.r_len:total] = new_v
             src_k, src_v = st.res_k, st.res_v
-        else:  # bulk prefill: larger than the window buffer, go through a temporary
+        elif from_empty:   # bulk prefill: the tokens are compressed from where they are
+            src_k, src_v = new_k, new_v
+        else:  # larger than the window buffer, go through a temporary
             src_k = torch.cat([st.res_k[:, :, : st.r_len], new_k], dim=2)
             src_v = torch.cat([st.res_v[:, :, : st.r_len], new_v], dim=2)
 
         if n_c > 0:
             st.reserve(st.n_comp + n_c)
             L = _lib.lib()
-            status = L.pare_kivi_append(
+            status = L.pare_kivi_append_kv(
                 src_k.data_ptr(), src_v.data_ptr(), _lib.dtype_code(st.dtype),
-                src_k.stride(0), src_k.stride(1), src_k.stride(2),
+                src_k.stride(0), src_k.stride(1), src_k.stride(2), src_v.stride(0), src_v.stride(1), src_v.stride(2),
                 n_c, st.n_comp, *st.cache_args(), *st.geometry(),
                 _lib.current_stream(st.device),
             )
-            _lib.check(status, "pare_kivi_append")
+            _lib.check(status, "pare_kivi_append_kv")
             st.n_comp += n_c
             keep_k = src_k[:, :, n_c:total]
             keep_v = src_v[:, :, n_c:total]
-            if src_k is st.res_k:  # shifting inside the same buffer: go through a copy
-                keep_k, keep_v = keep_k.clone(), keep_v.clone()
-            st.res_k[:, :, :r_after] = keep_k
-            st.res_v[:, :, :r_after] = keep_v
+            if defer_window and src_k is new_k:
+                left_k, left_v = keep_k, keep_v
+            else:
+                if src_k is st.res_k:  # shifting inside the same buffer: go through a copy
+                    keep_k, keep_v = keep_k.clone(), keep_v.clone()
+                st.res_k[:, :, :r_after] = keep_k
+                st.res_v[:, :, :r_after] = keep_v
         st.r_len = r_after
 
         self._compressed[layer_idx] = _CompressedKV(st) if st.n_comp > 0 else None
         self._residual_k[layer_idx] = st.res_k[:, :, : st.r_len]
         self._residual_v[layer_idx] = st.res_v[:, :, : st.r_len]
+        if defer_window:
+            return st, left_k, left_v
         return (st, deferred) if defer_single else st
 
     # ------------------------------------------------------------------ public API
     def update(self, layer_idx: int, new_k: Tensor, new_v: Tensor) -> tuple[Tensor, Tensor]:
         """Append ``[B, H, new_tokens, D]`` keys / values; return the dense ``(K, V)`` of the whole
         sequence in the input dtype (reference contract, ``pare/kv_cache.py:205-252``)."""
-        st = self._append(layer_idx, new_k, new_v)
+        st, left_k, left_v = self._append(layer_idx, new_k, new_v, defer_window=True)
         total = st.n_comp + st.r_len
         full_k = torch.empty(st.B, st.H, total, st.D, device=st.device, dtype=st.dtype)
         full_v = torch.empty_like(full_k)
+        if total == 0:
+            return full_k, full_v
+        n_left = 0 if left_k is None else left_k.shape[2]
+        n_old = st.r_len - n_left
+        code, stream = _lib.dtype_code(st.dtype), _lib.current_stream(st.device)
+        status = _lib.UNSUPPORTED
+        # one launch: reconstructed tokens, window, and the tokens that are on their way into the window
+        if not (st.res_k.requires_grad or st.res_v.requires_grad):
+            status = _lib.lib().pare_kivi_dense(
+                *st.cache_args(), *st.geometry(), st.n_comp,
+                full_k.data_ptr(), full_v.data_ptr(), code, full_k.stride(0), full_k.stride(1), full_k.stride(2),
+                st.res_k.data_ptr(), st.res_v.data_ptr(), st.res_k.stride(0), st.res_k.stride(1), st.res_k.stride(2), n_old,
+                *((left_k.data_ptr(), left_v.data_ptr(), left_k.stride(0), left_k.stride(1), left_k.stride(2),
+                   left_v.stride(0), left_v.stride(1), left_v.stride(2)) if n_left else (None, None, 0, 0, 0, 0, 0, 0)),
+                n_left, stream)
+        if status == 0:
+            return full_k, full_v
+        if status != _lib.UNSUPPORTED:
+            _lib.check(status, "pare_kivi_dense")
+        if n_left:
+            st.res_k[:, :, n_old:st.r_len] = left_k
+            st.res_v[:, :, n_old:st.r_len] = left_v
         if st.n_comp > 0:
             status = _lib.lib().pare_kivi_dequant(
                 *st.cache_args(), *st.geometry(), st.n_comp,
-                full_k.data_ptr(), full_v.data_ptr(), _lib.dtype_code(st.dtype),
-                full_k.stride(0), full_k.stride(1), full_k.stride(2),
-                _lib.current_stream(st.device),
+                full_k.data_ptr(), full_v.data_ptr(), code,
+                full_k.stride(0), full_k.stride(1), full_k.stride(2), stream,
             )
             _lib.check(status, "pare_kivi_dequant")
         full_k[:, :, st.n_comp:] = st.res_k[:, :, : st.r_len]
