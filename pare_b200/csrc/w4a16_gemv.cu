@@ -540,11 +540,24 @@ int launch_generic(const GemvParams& p, const uint8_t* packed, int G, cudaStream
 bool gemv_persist_supported(int M, int N, int K, int G, bool producer = false);
 size_t gemv_persist_partial_floats(int M, int N, int K);
 int gemv_persist_launch(const gemv::GemvParams& p, int x_dtype, cudaStream_t stream);
+bool gemv_tc_supported(int M, int N, int K, int G);
+size_t gemv_tc_partial_floats(int N, int K);
+int gemv_tc_launch(const gemv::GemvParams& p, int x_dtype, cudaStream_t stream);
 
 size_t prep_bytes(int M, int K) {  // prepared activations + step table, each rounded to 256 bytes
   const size_t xp = ((size_t)M * K * 2 + 255) / 256 * 256;
   const size_t tab = ((size_t)(K / 128 + 1) * kTabCols * sizeof(float4) + 255) / 256 * 256;
   return xp + tab;
+}
+
+// Which calls go to the tensor core as codes (w4a16_gemv_tc.cu): its time hardly depends on the rows, the streaming kernels'
+// grows with them.  Microseconds there / here, bf16: 9 rows 28672 x 4096 23.5 / 32.3, 4096 x 14336 15.3 / 32.1, 4096 x 4096
+// 8.0 / 9.0; 8 rows 28672 x 4096 23.5 / 26.3, 6144 x 4096 10.3 / 10.6, 4096 x 4096 7.8 / 7.5; 5 rows 4096 x 14336 14.8 /
+// 16.0, 8192 x 28672 43 / 57, 28672 x 4096 23.1 / 22.1 (above 8192 columns the streaming kernels cut K into slices).
+bool gemv_tc_rule(int M, int N, int K, int G) {
+  if (!gemv_tc_supported(M, N, K, G)) return false;
+  const bool large = (int64_t)N * K >= (int64_t)24 << 20;
+  return M >= 9 || (M >= 7 && large) || (M >= 5 && large && K > 8192);
 }
 
 size_t gemv_workspace_bytes(int M, int N, int K, int G) {
@@ -553,7 +566,12 @@ size_t gemv_workspace_bytes(int M, int N, int K, int G) {
   if (K % 256 == 0 && G % 128 == 0) splits = (size_t)(K / 256);  // upper bound on any plan
   if (splits > 64) splits = 64;
   // split-K partial sums of either schedule (the persistent one adds at most one 32-row block per SM)
-  return kCounterBytes + prep_bytes(m, K) + (splits * (size_t)m * N + (size_t)sm_count() * 32 * m) * sizeof(float);
+  size_t floats = splits * (size_t)m * N + (size_t)sm_count() * 32 * m;
+  if (gemv_tc_rule(m, N, K, G)) {
+    const size_t t = gemv_tc_partial_floats(N, K);
+    if (t > floats) floats = t;
+  }
+  return kCounterBytes + prep_bytes(m, K) + floats * sizeof(float);
 }
 
 // Called by pare_w4a16_forward for every chunk of at most 16 activation rows.
@@ -603,9 +621,11 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   PARE_REQUIRE((pl.steps_per_split + pl.warps - 1) / pl.warps <= kMaxStepsPerWarp / pl.rb, PARE_ERR_UNSUPPORTED);
   p.splits = pl.splits;
   p.steps_per_split = pl.steps_per_split;
+  const bool tensor = !prod && !peer && scale && zero && !meta_h2 && gemv_tc_rule(M, N, K, G);
   const bool persist = gemv_persist_supported(M, N, K, G, prod != nullptr);
   const size_t need = kCounterBytes + prep_bytes(M, K) +
-                      (persist ? gemv_persist_partial_floats(M, N, K) * sizeof(float)
+                      (tensor ? gemv_tc_partial_floats(N, K) * sizeof(float) :
+                       persist ? gemv_persist_partial_floats(M, N, K) * sizeof(float)
                                : (pl.splits > 1 ? (size_t)pl.splits * M * N * sizeof(float) : 0));
   PARE_REQUIRE(workspace != nullptr && workspace_bytes >= need, PARE_ERR_WORKSPACE);
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
@@ -642,6 +662,7 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
                                               : cudaLaunchKernelEx(&cfg, w4a16_prep_kernel<__nv_bfloat16>, p);
     if (e != cudaSuccess) return PARE_ERR_CUDA;
   }
+  if (tensor) return gemv_tc_launch(p, x_dtype, stream);
   // 2) the streaming kernel: persistent schedule for large layers at M <= 4, one tile per CTA otherwise
   if (persist) return gemv_persist_launch(p, x_dtype, stream);
   return x_dtype == PARE_F16 ? dispatch_gemv<__half>(p, pl, stream) : dispatch_gemv<__nv_bfloat16>(p, pl, stream);
