@@ -253,9 +253,7 @@ class DecodeStack(nn.Module):
                     resid, spare = spare, resid
             else:
                 qkv = blk.qkv(self._rmsnorm(resid, delta, blk.norm1, store_residual=delta is not None))
-            q = qkv[:, : hq * d].unflatten(1, (hq, d))
-            k = qkv[:, hq * d:(hq + hkv) * d].unflatten(1, (hkv, 1, d))
-            v = qkv[:, (hq + hkv) * d:].unflatten(1, (hkv, 1, d))
+            q, k, v = qkv.view(m, hq + 2 * hkv, 1, d).split((hq, hkv, hkv), dim=1)      # [M, heads, 1, d] views
             if fused:
                 self.cache.attend(i, q, k, v, scale=1.0 / math.sqrt(d), prepared_out=p_attn, rope=rope)
                 # tensor parallel: the sums of the two row-parallel layers over the ranks are added inside their kernels

@@ -8,6 +8,7 @@ with it.  Signatures mirror ``include/pare_b200.h`` one to one.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import threading
 from pathlib import Path
 
@@ -126,8 +127,21 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def _index(device: torch.device) -> int:
+    index = device.index
+    return torch.cuda.current_device() if index is None else index
+
+
 def current_stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the current stream of ``device`` (the raw handle: a ``torch.cuda.Stream`` object per launch costs more
+    than some of the launches)."""
+    return torch._C._cuda_getCurrentRawStream(_index(device))
+
+
+@functools.lru_cache(maxsize=1024)
+def w4a16_workspace_bytes(m: int, n: int, k: int, group_size: int) -> int:
+    """``pare_w4a16_workspace_bytes``: a function of the sizes alone, remembered for the shapes in use."""
+    return lib().pare_w4a16_workspace_bytes(m, n, k, group_size)
 
 
 # One zero-initialised workspace per device and stream; the kernels leave it zero-consistent.
@@ -137,18 +151,17 @@ _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 def workspace_status(device: torch.device) -> int:
     """Status word of the current stream's workspace on ``device``: 0, or the time-out code if a bounded wait inside a
     kernel gave up since the last read.  Synchronises the stream and clears the word; 0 if no workspace exists yet."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+    key = (_index(device), current_stream(device))
     buf = _workspaces.get(key)
     if buf is None:
         return 0
-    return lib().pare_workspace_status(buf.data_ptr(), current_stream(device))
+    return lib().pare_workspace_status(buf.data_ptr(), key[1])
 
 
-def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Zero-filled scratch buffer of at least ``nbytes`` for the current stream of ``device``."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+def workspace(device: torch.device, nbytes: int, stream: int | None = None) -> torch.Tensor:
+    """Zero-filled scratch buffer of at least ``nbytes`` for the current stream of ``device`` (``stream``: its handle, where
+    the caller has it already)."""
+    key = (_index(device), current_stream(device) if stream is None else stream)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         size = max(nbytes, 8 << 20)

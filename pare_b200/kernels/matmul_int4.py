@@ -83,24 +83,24 @@ def w4a16_forward(
     assert packed_weight.dtype == torch.uint8 and packed_weight.is_contiguous()
     if m == 0:
         return x.new_empty(0, n)
-    code = _lib.dtype_code(x.dtype)
-    if bias is not None and bias.dtype != x.dtype:
-        bias = bias.to(x.dtype)
-    y = out if out is not None else torch.empty(m, n, device=x.device, dtype=x.dtype)
-    L = _lib.lib()
-    ws_bytes = L.pare_w4a16_workspace_bytes(m, n, k, group_size)
-    ws = _lib.workspace(x.device, ws_bytes)
-    status = L.pare_w4a16_forward(
+    dtype, dev = x.dtype, x.device
+    code = _lib.dtype_code(dtype)
+    if bias is not None and bias.dtype != dtype:
+        bias = bias.to(dtype)
+    y = out if out is not None else torch.empty(m, n, device=dev, dtype=dtype)
+    stream = _lib.current_stream(dev)
+    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size), stream)
+    status = _lib.lib().pare_w4a16_forward(
         x.data_ptr(), code, x.stride(0),
         packed_weight.data_ptr(),
         _lib.ptr(scale), _lib.ptr(zero), _lib.ptr(meta_h2),
         _lib.ptr(col_perm), _lib.ptr(input_scale), _lib.ptr(bias),
         y.data_ptr(), y.stride(0),
         m, n, k, group_size,
-        ws.data_ptr(), ws.numel(),
-        _lib.current_stream(x.device),
+        ws.data_ptr(), ws.numel(), stream,
     )
-    _lib.check(status, "pare_w4a16_forward")
+    if status:
+        _lib.check(status, "pare_w4a16_forward")
     return y
 
 
@@ -150,19 +150,20 @@ def w4a16_forward_prepared(prep: PreparedActivations, packed_weight: Tensor, sca
     dev = packed_weight.device
     y = out if out is not None else torch.empty(m, n, device=dev, dtype=prep.dtype)
     L = _lib.lib()
-    ws = _lib.workspace(dev, L.pare_w4a16_workspace_bytes(m, n, k, group_size))
+    stream = _lib.current_stream(dev)
+    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size), stream)
     if peer is not None:
         status = L.pare_w4a16_forward_prepared_allreduce(
             prep.data_ptr(), _lib.dtype_code(prep.dtype), packed_weight.data_ptr(),
             _lib.ptr(scale), _lib.ptr(zero), _lib.ptr(meta_h2), _lib.ptr(bias),
             y.data_ptr(), y.stride(0), m, n, k, group_size, ws.data_ptr(), ws.numel(),
-            peer.rank, peer.world, peer._ptrs, peer.buffer_bytes, _lib.current_stream(dev))
+            peer.rank, peer.world, peer._ptrs, peer.buffer_bytes, stream)
         _lib.check(status, "pare_w4a16_forward_prepared_allreduce")
         return y
     status = L.pare_w4a16_forward_prepared(
         prep.data_ptr(), _lib.dtype_code(prep.dtype), packed_weight.data_ptr(),
         _lib.ptr(scale), _lib.ptr(zero), _lib.ptr(meta_h2), _lib.ptr(bias),
-        y.data_ptr(), y.stride(0), m, n, k, group_size, ws.data_ptr(), ws.numel(), _lib.current_stream(dev))
+        y.data_ptr(), y.stride(0), m, n, k, group_size, ws.data_ptr(), ws.numel(), stream)
     _lib.check(status, "pare_w4a16_forward_prepared")
     return y
 
@@ -192,19 +193,21 @@ def w4a16_forward_produced(producer: int, a: Tensor, packed_weight: Tensor, scal
         bias = bias.to(a.dtype)
     y = out if out is not None else torch.empty(m, n, device=a.device, dtype=a.dtype)
     L = _lib.lib()
-    ws = _lib.workspace(a.device, L.pare_w4a16_workspace_bytes(m, n, k, group_size))
+    dev = a.device
+    stream = _lib.current_stream(dev)
+    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size), stream)
     if peer is not None:   # row-parallel shard: the sum over the ranks is added inside the kernel
         status = L.pare_w4a16_forward_produced_allreduce(
             producer, a.data_ptr(), _lib.ptr(delta), _lib.ptr(norm_weight), _lib.ptr(resid_out), a.stride(0), float(eps),
             _lib.dtype_code(a.dtype), packed_weight.data_ptr(), _lib.ptr(scale), _lib.ptr(zero), _lib.ptr(meta_h2), _lib.ptr(bias),
             y.data_ptr(), y.stride(0), m, n, k, group_size, ws.data_ptr(), ws.numel(),
-            peer.rank, peer.world, peer._ptrs, peer.buffer_bytes, _lib.current_stream(a.device))
+            peer.rank, peer.world, peer._ptrs, peer.buffer_bytes, stream)
         _lib.check(status, "pare_w4a16_forward_produced_allreduce")
         return y
     status = L.pare_w4a16_forward_produced(
         producer, a.data_ptr(), _lib.ptr(delta), _lib.ptr(norm_weight), _lib.ptr(resid_out), a.stride(0), float(eps),
         _lib.dtype_code(a.dtype), packed_weight.data_ptr(), _lib.ptr(scale), _lib.ptr(zero), _lib.ptr(meta_h2), _lib.ptr(bias),
-        y.data_ptr(), y.stride(0), m, n, k, group_size, ws.data_ptr(), ws.numel(), _lib.current_stream(a.device))
+        y.data_ptr(), y.stride(0), m, n, k, group_size, ws.data_ptr(), ws.numel(), stream)
     _lib.check(status, "pare_w4a16_forward_produced")
     return y
 

@@ -176,6 +176,9 @@ class _LayerStore:
         return (self.k_codes.data_ptr(), self.k_scale.data_ptr(), self.k_zero.data_ptr(),
                 self.v_codes.data_ptr(), self.v_scale.data_ptr(), self.v_zero.data_ptr())
 
+    def window_args(self) -> tuple:
+        return (self.res_k.data_ptr(), self.res_v.data_ptr(), *self.res_k.stride()[:3])
+
     def geometry(self) -> tuple:
         return (self.B, self.H, self.D, self.cfg.bits, self.cfg.group_size, self.v_group, self.cap)
 
@@ -282,18 +285,18 @@ class QuantizedKVCache:
         n_c, r_after = plan_update(st.r_len, n_new, cfg.residual_length, cfg.group_size)
         total = st.r_len + n_new
 
-        deferred = (defer_single and n_new == 1 and n_c == 0 and total <= st.r_cap
-                    and new_k.data_ptr() % 16 == 0 and new_v.data_ptr() % 16 == 0
-                    and all(t.stride(3) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 for t in (new_k, new_v))
-                    and new_k.stride() == new_v.stride())
+        deferred = False
+        if defer_single and n_new == 1 and n_c == 0 and total <= st.r_cap and new_k.data_ptr() % 16 == 0 and new_v.data_ptr() % 16 == 0:
+            strides = new_k.stride()
+            deferred = strides[3] == 1 and strides[0] % 8 == 0 and strides[1] % 8 == 0 and new_v.stride() == strides
         if rope is not None and not deferred:   # the kernel rotates only a key it appends itself
             new_k = apply_rope(new_k, rope)
         left_k = left_v = None   # with defer_window: what the caller copies into the window
         # kernels may read the new tokens where they are: same device and dtype as the store, nothing for autograd to see
-        plain = (new_k.device == st.device and new_v.device == st.device and new_v.dtype == st.dtype
-                 and new_k.stride(3) == 1 and new_v.stride(3) == 1
-                 and not (torch.is_grad_enabled() and (new_k.requires_grad or new_v.requires_grad)))
-        from_empty = st.r_len == 0 and plain
+        plain = not deferred and (new_k.device == st.device and new_v.device == st.device and new_v.dtype == st.dtype
+                                  and new_k.stride(3) == 1 and new_v.stride(3) == 1
+                                  and not (torch.is_grad_enabled() and (new_k.requires_grad or new_v.requires_grad)))
+        from_empty = plain and st.r_len == 0
         if deferred:
             pass
         elif total <= st.r_cap:
@@ -331,9 +334,10 @@ class QuantizedKVCache:
                 st.res_v[:, :, :r_after] = keep_v
         st.r_len = r_after
 
-        self._compressed[layer_idx] = _CompressedKV(st) if st.n_comp > 0 else None
-        self._residual_k[layer_idx] = st.res_k[:, :, : st.r_len]
-        self._residual_v[layer_idx] = st.res_v[:, :, : st.r_len]
+        if st.n_comp > 0 and self._compressed[layer_idx] is None:
+            self._compressed[layer_idx] = _CompressedKV(st)
+        self._residual_k[layer_idx] = st.res_k.narrow(2, 0, st.r_len)
+        self._residual_v[layer_idx] = st.res_v.narrow(2, 0, st.r_len)
         if defer_window:
             return st, left_k, left_v
         return (st, deferred) if defer_single else st
@@ -404,34 +408,33 @@ class QuantizedKVCache:
         st, fused_new = self._append(layer_idx, new_k, new_v, defer_single=True, rope=rope)
         if q.dtype != st.dtype:
             raise ValueError("attend() needs q in the cache dtype")
-        q3 = q.reshape(q.shape[0], q.shape[1], q.shape[-1])
-        if q3.stride(-1) != 1:
-            q3 = q3.contiguous()
-        B, Hq, D = q3.shape
+        shape = q.shape
+        if q.dim() != 4 or q.shape[2] != 1 or q.stride(3) != 1:
+            q = q.reshape(q.shape[0], q.shape[1], 1, q.shape[-1])
+            if q.stride(3) != 1:
+                q = q.contiguous()
+        B, Hq, _, D = q.shape
         out = None if prepared_out is not None else torch.empty(B, Hq, D, device=q.device, dtype=q.dtype)
         if prepared_out is not None and (prepared_out.rows, prepared_out.k, prepared_out.dtype) != (B, Hq * D, q.dtype):
             raise ValueError("prepared_out does not match the attention output")
-        nk = nv = None
-        if fused_new:
-            nk, nv = new_k[:, :, 0], new_v[:, :, 0]     # [B, H, D] views
-            if nk.stride(-1) != 1 or nv.stride() != nk.stride():
-                nk, nv = nk.contiguous(), nv.contiguous()
         L = _lib.lib()
-        ws = _lib.workspace(st.device, L.pare_kivi_attn_workspace_bytes(B, st.H, st.n_comp, st.r_len))
+        stream = _lib.current_stream(st.device)
+        ws = _lib.workspace(st.device, L.pare_kivi_attn_workspace_bytes(B, st.H, st.n_comp, st.r_len), stream)
         status = L.pare_kivi_decode_attn(
-            q3.data_ptr(), _lib.dtype_code(q.dtype), q3.stride(0), q3.stride(1),
+            q.data_ptr(), _lib.dtype_code(q.dtype), q.stride(0), q.stride(1),
             *st.cache_args(), st.n_comp,
-            st.res_k.data_ptr(), st.res_v.data_ptr(), st.res_k.stride(0), st.res_k.stride(1), st.res_k.stride(2), st.r_len,
-            _lib.ptr(nk), _lib.ptr(nv), nk.stride(0) if fused_new else 0, nk.stride(1) if fused_new else 0,
+            *st.window_args(), st.r_len,
+            # the new token where it is, if the kernel is to append it: [B, H, 1, D], channels contiguous, equal strides
+            *((new_k.data_ptr(), new_v.data_ptr(), new_k.stride(0), new_k.stride(1)) if fused_new else (None, None, 0, 0)),
             _lib.ptr(rope),
-            _lib.ptr(out), out.stride(0) if out is not None else 0, out.stride(1) if out is not None else 0,
+            *((None, 0, 0) if out is None else (out.data_ptr(), Hq * D, D)),
             prepared_out.data_ptr() if prepared_out is not None else None,
             float(scale if scale is not None else 1.0 / math.sqrt(D)),
             B, Hq, st.H, D, self.config.bits, self.config.group_size, st.v_group, st.cap,
-            ws.data_ptr(), ws.numel(), _lib.current_stream(st.device),
+            ws.data_ptr(), ws.numel(), stream,
         )
         _lib.check(status, "pare_kivi_decode_attn")
-        return None if out is None else out.reshape(q.shape)
+        return None if out is None else out.reshape(shape)
 
     def prefill(self, layer_idx: int, q: Tensor, new_k: Tensor, new_v: Tensor, scale: float | None = None,
                 rope: Tensor | None = None) -> Tensor:

@@ -40,6 +40,7 @@ from pare_b200.core.dtype import QuantDtype
 from pare_b200.core.functional import dequantize_tensor, quantize_tensor
 from pare_b200.core.pack import pack_int4, unpack_int4
 from pare_b200.core.scale import compute_scale
+from pare_b200.kernels import matmul_int4 as _matmul
 
 _FP8 = (QuantDtype.FP8_E4M3, QuantDtype.FP8_E5M2)
 
@@ -149,36 +150,42 @@ class QuantizedLinear(nn.Module):
         self.register_buffer("_zero_kernel", zero2d, persistent=False)
         self.register_buffer("_meta_h2_kernel", pack_meta_h2(scale2d, zero2d), persistent=False)
 
-    def _forward_kernel(self, x: Tensor) -> Tensor:
-        from pare_b200.kernels.matmul_int4 import w4a16_forward
-
-        if not hasattr(self, "_packed_weight_kernel"):
+    # A decode projection takes a few microseconds on the GPU, so the way there counts: buffers by their dictionary (an
+    # nn.Module attribute that is a buffer is found only after two failed lookups), no-op reshapes and casts left out.
+    def _kernel_buffers(self) -> dict:
+        bufs = self._buffers
+        if "_packed_weight_kernel" not in bufs:
             self._prepare_kernel_buffers()
-        shape = x.shape
-        out_dtype = x.dtype
-        x2d = x.reshape(-1, self.in_features)
-        if x2d.dtype not in (torch.float16, torch.bfloat16):
+        return bufs
+
+    def _forward_kernel(self, x: Tensor) -> Tensor:
+        bufs = self._kernel_buffers()
+        dtype, flat = x.dtype, x.dim() == 2
+        x2d = x if flat and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
+        if dtype is not torch.float16 and dtype is not torch.bfloat16:
             x2d = x2d.to(torch.float16)
-        if x2d.stride(-1) != 1:
+        if x2d.stride(1) != 1:
             x2d = x2d.contiguous()
         use_h2 = self.kernel_meta_fp16
-        y = w4a16_forward(
+        y = _matmul.w4a16_forward(
             x2d,
-            self._packed_weight_kernel,
-            None if use_h2 else self._scale_kernel,
-            None if use_h2 else self._zero_kernel,
+            bufs["_packed_weight_kernel"],
+            None if use_h2 else bufs["_scale_kernel"],
+            None if use_h2 else bufs["_zero_kernel"],
             self._kernel_group_size(),
             bias=self.bias,
-            col_perm=self._col_perm_kernel,
+            col_perm=bufs["_col_perm_kernel"],
             input_scale=self.input_scale,
-            meta_h2=self._meta_h2_kernel if use_h2 else None,
+            meta_h2=bufs["_meta_h2_kernel"] if use_h2 else None,
         )
-        return y.to(out_dtype).reshape(*shape[:-1], self.out_features)
+        if y.dtype is not dtype:
+            y = y.to(dtype)
+        return y if flat else y.reshape(*x.shape[:-1], self.out_features)
 
     def supports_prepared(self, rows: int) -> bool:
         """True if :meth:`forward_prepared` can serve ``rows`` activation rows of this layer."""
-        return (self.use_kernel and self.config.dtype == QuantDtype.INT4 and not self.quantize_inputs
-                and self.g_idx is None and self.input_scale is None and rows <= 16
+        return (rows <= 16 and self.use_kernel and self.config.dtype == QuantDtype.INT4 and not self.quantize_inputs
+                and self.g_idx is None and self.input_scale is None
                 and self.in_features % 256 == 0 and self._kernel_group_size() % 128 == 0)
 
     def forward_prepared(self, prep, peer=None) -> Tensor:
@@ -186,30 +193,22 @@ class QuantizedLinear(nn.Module):
         the producing kernel wrote them in operand order, so no preparation launch is needed.  ``peer`` (a
         ``PeerAllReduce``): this layer is a row-parallel shard; the result is the sum over the ranks, added inside
         the kernel."""
-        from pare_b200.kernels.matmul_int4 import w4a16_forward_prepared
-
         if not self.supports_prepared(prep.rows):
             raise ValueError("this layer cannot take prepared activations (act-order, input scale, shape or row count)")
-        if not hasattr(self, "_packed_weight_kernel"):
-            self._prepare_kernel_buffers()
-        use_h2 = self.kernel_meta_fp16
-        return w4a16_forward_prepared(
-            prep, self._packed_weight_kernel,
-            None if use_h2 else self._scale_kernel, None if use_h2 else self._zero_kernel,
-            self._kernel_group_size(), bias=self.bias, meta_h2=self._meta_h2_kernel if use_h2 else None, peer=peer)
+        bufs, use_h2 = self._kernel_buffers(), self.kernel_meta_fp16
+        return _matmul.w4a16_forward_prepared(
+            prep, bufs["_packed_weight_kernel"],
+            None if use_h2 else bufs["_scale_kernel"], None if use_h2 else bufs["_zero_kernel"],
+            self._kernel_group_size(), bias=self.bias, meta_h2=bufs["_meta_h2_kernel"] if use_h2 else None, peer=peer)
 
     def _forward_produced(self, producer: int, a: Tensor, **kw) -> Tensor:
-        from pare_b200.kernels.matmul_int4 import w4a16_forward_produced
-
         if not self.supports_prepared(a.shape[0]):
             raise ValueError("this layer cannot compute its activations in-kernel (act-order, input scale, shape or row count)")
-        if not hasattr(self, "_packed_weight_kernel"):
-            self._prepare_kernel_buffers()
-        use_h2 = self.kernel_meta_fp16
-        return w4a16_forward_produced(
-            producer, a, self._packed_weight_kernel,
-            None if use_h2 else self._scale_kernel, None if use_h2 else self._zero_kernel,
-            self._kernel_group_size(), bias=self.bias, meta_h2=self._meta_h2_kernel if use_h2 else None, **kw)
+        bufs, use_h2 = self._kernel_buffers(), self.kernel_meta_fp16
+        return _matmul.w4a16_forward_produced(
+            producer, a, bufs["_packed_weight_kernel"],
+            None if use_h2 else bufs["_scale_kernel"], None if use_h2 else bufs["_zero_kernel"],
+            self._kernel_group_size(), bias=self.bias, meta_h2=bufs["_meta_h2_kernel"] if use_h2 else None, **kw)
 
     def forward_rmsnorm(self, x: Tensor, delta: Tensor | None, norm_weight: Tensor, resid_out: Tensor | None = None,
                         eps: float = 1e-5) -> Tensor:
