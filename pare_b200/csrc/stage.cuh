@@ -11,6 +11,7 @@
 namespace pare {
 namespace gemv {
 
+constexpr int kProducerPlain = 16;   // activations as they are (a = x [M][lda], no gather, no input scale): only brought into operand order
 constexpr int kStageRounds = 4;   // most steps a half warp of the staging threads takes: K <= 128 * rounds * threads / 16
 
 // Norm weights of the steps a thread will produce: constants of the model, so they can be fetched before
@@ -93,7 +94,7 @@ __device__ __forceinline__ void stage_produce(const GemvParams& p, int st0, int 
       }
     }
   } else {
-    // y = silu(gate) * up, gate = a[m][k], up = a[m][K + k]; any K range
+    // y = silu(gate) * up, gate = a[m][k], up = a[m][K + k], or y = a; any K range
     for (int m = 0; m < p.M; ++m) {
       for (int r0 = 0; r0 < nst; r0 += n_hw) {
         const int sl = r0 + hw;   // step within the range
@@ -102,13 +103,18 @@ __device__ __forceinline__ void stage_produce(const GemvParams& p, int st0, int 
         if (live) {
           const size_t off = (size_t)m * p.lda + (size_t)(st0 + sl) * 128 + c * 8;
           const uint4 gv = *reinterpret_cast<const uint4*>(a + off);
-          const uint4 uv = *reinterpret_cast<const uint4*>(a + off + p.K);
           const T* ge = reinterpret_cast<const T*>(&gv);
-          const T* ue = reinterpret_cast<const T*>(&uv);
+          if (p.producer == kProducerPlain) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float g = to_float<T>(ge[e]);
-            o[e] = g / (1.f + __expf(-g)) * to_float<T>(ue[e]);
+            for (int e = 0; e < 8; ++e) o[e] = to_float<T>(ge[e]);
+          } else {
+            const uint4 uv = *reinterpret_cast<const uint4*>(a + off + p.K);
+            const T* ue = reinterpret_cast<const T*>(&uv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float g = to_float<T>(ge[e]);
+              o[e] = g / (1.f + __expf(-g)) * to_float<T>(ue[e]);
+            }
           }
         }
         prep_store_step<T>(o, live, reinterpret_cast<__half*>(xs + (size_t)m * xstride) + sl * 128, c,

@@ -621,7 +621,21 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   PARE_REQUIRE((pl.steps_per_split + pl.warps - 1) / pl.warps <= kMaxStepsPerWarp / pl.rb, PARE_ERR_UNSUPPORTED);
   p.splits = pl.splits;
   p.steps_per_split = pl.steps_per_split;
-  const bool tensor = !prod && !peer && scale && zero && !meta_h2 && gemv_tc_rule(M, N, K, G);
+  // Up to four rows that need no gather and no input scale are brought into operand order by the streaming kernel itself, like
+  // the outputs of the fused producers: a few KB from L2 per CTA instead of a launch of their own.  Not where many small
+  // tiles would each do it, nor for the largest layers' three or four rows (one call, microseconds with / without the
+  // launch: 4096 x 4096 1 row 6.5 / 5.1, 28672 x 4096 18.3 / 17.3, 3584 x 18944 15.0 / 13.3, 1024 x 4096 4 rows 7.6 / 6.8;
+  // 6144 x 4096, 384 tiles, 1 row 6.9 / 8.8; 57344 x 8192, 4 rows 77 / 80).
+  if (!prod && !prepared && !peer && M <= 4 && pl.fast && col_perm == nullptr && input_scale == nullptr && p.x_vec_ok) {
+    const bool few = gemv_persist_supported(M, N, K, G) ? M <= 2 || (int64_t)N * K <= (int64_t)1 << 27
+                                                        : (int64_t)((N + 16 * pl.rb - 1) / (16 * pl.rb)) * pl.splits <= 2 * sm_count();
+    if (few) {
+      p.producer = kProducerPlain;
+      p.pa = x;
+      p.lda = ldx;
+    }
+  }
+  const bool tensor = !p.producer && !peer && scale && zero && !meta_h2 && gemv_tc_rule(M, N, K, G);
   const bool persist = gemv_persist_supported(M, N, K, G, prod != nullptr);
   const size_t need = kCounterBytes + prep_bytes(M, K) +
                       (tensor ? gemv_tc_partial_floats(N, K) * sizeof(float) :
@@ -648,7 +662,7 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
     }
   }
   // 1) activations into operand order (one warp per row and 128-column step)
-  if (!prepared && !prod) {
+  if (!prepared && !p.producer) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((M * (K / 128) + 7) / 8, 1, 1);
     cfg.blockDim = dim3(128, 1, 1);
