@@ -70,16 +70,30 @@ struct GemmParams {
 // ---- activations for the tensor-core path when they need work: the act-order gather and / or the run-time input
 // scale, into a dense [M][K] copy in column order.  Plain layers skip this launch: the activation tiles are then
 // fetched by TMA straight from the caller's tensor. ----
+// Eight columns per thread: their sources and scales in two or four 16-byte loads, all eight gathers in flight, one
+// 16-byte store.  (A column per thread and a 64-bit division each took 5 us for 64 x 14336.)
 template <typename T>
-__global__ void w4a16_gemm_prep_kernel(const T* x, int64_t ldx, const int32_t* col_perm, const float* input_scale, T* xq,
-                                       int M, int K) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)M * K) return;
-  const int m = (int)(idx / K), k = (int)(idx - (int64_t)m * K);
-  const int src = col_perm ? col_perm[k] : k;
-  float v = to_float<T>(x[(int64_t)m * ldx + src]);
-  if (input_scale) v = __fdiv_rn(v, input_scale[src]);
-  xq[(int64_t)m * K + k] = from_float<T>(v);
+__global__ void __launch_bounds__(128) w4a16_gemm_prep_kernel(const T* x, int64_t ldx, const int32_t* col_perm, const float* input_scale, T* xq,
+                                                              int K) {
+  const int k = (blockIdx.y * 128 + threadIdx.x) * 8, m = blockIdx.x;
+  if (k >= K) return;   // K % 8 == 0
+  const T* row = x + (int64_t)m * ldx;
+  int src[8];
+  if (col_perm && (reinterpret_cast<uintptr_t>(col_perm) & 15u) == 0) {
+    const int4 a = __ldg(reinterpret_cast<const int4*>(col_perm + k)), b = __ldg(reinterpret_cast<const int4*>(col_perm + k + 4));
+    src[0] = a.x; src[1] = a.y; src[2] = a.z; src[3] = a.w; src[4] = b.x; src[5] = b.y; src[6] = b.z; src[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) src[i] = col_perm ? __ldg(col_perm + k + i) : k + i;
+  }
+  T v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = row[src[i]];
+  if (input_scale) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = from_float<T>(__fdiv_rn(to_float<T>(v[i]), __ldg(input_scale + src[i])));
+  }
+  *reinterpret_cast<uint4*>(xq + (int64_t)m * K + k) = *reinterpret_cast<const uint4*>(v);
 }
 
 // Packed fp32 pairs (two independent IEEE operations per instruction).
@@ -145,10 +159,10 @@ __device__ __forceinline__ void dequant_word(uint32_t w, const DqConst& c, uint3
 // What bounds it, and why this shape (one B200, bf16): with the dequantized weights in shared memory that memory had to
 // carry 208 KB per 128 columns at 256 activation rows (weights written and read, activations written and read, codes), 1.6
 // times what it moves in the 1024 cycles of the MMAs.  With the weights in tensor memory 144 KB remain, and the freed 64 KB
-// hold one more activation stage.  Few rows are bound by the dequantizing warps (about 900 cycles per 128 columns);
+// hold one more activation stage.  Few rows are bound by the dequantizing warps (about 750 cycles per 128 columns);
 // four stages instead of two keep the MMA's round trip off their path, and equal runs of units instead of whole tiles per
-// CTA keep all SMs busy to the end.  28672 x 4096: 64 rows 65.9 -> 40.0 us, 256 rows 74.5 -> 61.0, 2048 rows 473 -> 393 us
-// (1225 TFLOP/s); 4096 x 4096: 64 rows 23.6 -> 15.2, 128 rows 35.0 -> 18.3; 3584 x 18944, 1531 rows 294 -> 184 us.
+// CTA keep all SMs busy to the end.  28672 x 4096: 64 rows 65.9 -> 36.6 us, 256 rows 74.5 -> 59.4, 2048 rows 473 -> 395 us
+// (1217 TFLOP/s); 4096 x 4096: 64 rows 23.6 -> 14.9, 128 rows 35.0 -> 17.2; 3584 x 18944, 1531 rows 294 -> 188 us.
 template <typename T>
 __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                                                                     const GemmParams p) {
@@ -204,18 +218,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
     const uint32_t a_dst = tmem + kTmemA + ((uint32_t)((warp & 3) * 32) << 16) + grp * 32;
     float sc[2], zc[2], sc_n[2], zc_n[2];
     // scale / zero of a unit's two stages: a row-strided (one line per thread) read that often comes from DRAM, so the
-    // next unit's values are requested a whole unit before they are needed
-    auto load_meta = [&](int u) {
-      const int t = u / ku, k = u - t * ku;
-      const size_t row = (size_t)min((t / p.mtiles) * kRows + r, p.N - 1) * p.ngroups;
+    // next unit's values are requested a whole unit before they are needed.  Position of the next request, kept by
+    // counting: the divisions that derive it from the unit's number cost a third of a unit's dequantization.
+    int mt = u0 / ku, mk = u0 - mt * ku, mw = mt / p.mtiles, mm = mt - mw * p.mtiles, mg = 2 * mk / spg, mr = 2 * mk - mg * spg;
+    size_t mrow = (size_t)min(mw * kRows + r, p.N - 1) * p.ngroups;
+    auto load_meta = [&] {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int g = (2 * k + i) / spg;
-        sc_n[i] = __ldg(p.scale + row + g);
-        zc_n[i] = __ldg(p.zero + row + g);
+        sc_n[i] = __ldg(p.scale + mrow + mg);
+        zc_n[i] = __ldg(p.zero + mrow + mg);
+        if (++mr == spg) mr = 0, ++mg;
+      }
+      if (++mk == ku) {
+        mk = mg = mr = 0;
+        if (++mm == p.mtiles) mm = 0, ++mw;
+        mrow = (size_t)min(mw * kRows + r, p.N - 1) * p.ngroups;
       }
     };
-    load_meta(u0);
+    load_meta();
     int slot = 0, s = 0;
     uint32_t rpar = 0, spar = 1;
     for (int u = u0; u < u1; ++u) {
@@ -224,7 +244,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
         sc[i] = sc_n[i];
         zc[i] = zc_n[i];
       }
-      if (u + 1 < u1) load_meta(u + 1);
+      if (u + 1 < u1) load_meta();
       bar_wait(raw_full + slot * 8, rpar, status, dead);
       const uint32_t raw_row = raw + slot * kRawBytes + r * 128;
 #pragma unroll
@@ -550,13 +570,12 @@ int gemm_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   //    described by a tensor map: 16-byte aligned base and row pitch), otherwise used where they are
   const bool direct = col_perm == nullptr && input_scale == nullptr && aligned16(x) && (ldx % 8) == 0;
   if (!direct) {
-    const int64_t total = (int64_t)M * K;
-    const unsigned blocks = (unsigned)((total + 255) / 256);
+    const dim3 blocks(M, (K / 8 + 127) / 128);
     if (x_dtype == PARE_F16)
-      w4a16_gemm_prep_kernel<__half><<<blocks, 256, 0, stream>>>((const __half*)x, ldx, col_perm, input_scale, (__half*)xq, M, K);
+      w4a16_gemm_prep_kernel<__half><<<blocks, 128, 0, stream>>>((const __half*)x, ldx, col_perm, input_scale, (__half*)xq, K);
     else
-      w4a16_gemm_prep_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)x, ldx, col_perm, input_scale,
-                                                                        (__nv_bfloat16*)xq, M, K);
+      w4a16_gemm_prep_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>((const __nv_bfloat16*)x, ldx, col_perm, input_scale,
+                                                                        (__nv_bfloat16*)xq, K);
     if (cudaGetLastError() != cudaSuccess) return PARE_ERR_CUDA;
   }
 
