@@ -7,7 +7,7 @@
 // every instruction:   Y^T[n][m] = sum_k W[n][k] * X[m][k].
 //
 // A persistent grid, one CTA per SM.  The work is the list of (128-row weight tile, activation tile, 256-column unit)
-// in that nesting order; a CTA takes one contiguous run of units, so a run may begin and end inside a tile.  Tiles that
+// in that nesting order (the first two exchanged for very large activations); a CTA takes one contiguous run of units, so a run may begin and end inside a tile.  Tiles that
 // lie in several runs are finished by the CTA that arrives last, which adds the fp32 partial sums in K order.
 // Warp roles:
 //   warps 0-7    dequantize (two groups of four warps, one per 64-column block of a 128-column stage, one thread per
@@ -58,7 +58,8 @@ struct GemmParams {
   int64_t ldy;
   int M, N, K, ngroups, group_size;
   int mt;               // activation rows per tile (UMMA N): a multiple of 16, 32 .. 256
-  int mtiles;           // activation tiles
+  int inner;            // tiles of the inner direction of the tile order
+  int rows_inner;       // 1: weight tiles are the inner direction (activation tiles the outer), 0: the other way round
   int tile_units;       // units per tile: K / 256
   int total_units;      // units of the whole product
   int run_units;        // units per CTA
@@ -180,6 +181,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform, and known to be
   const int ku = p.tile_units;
   const int u0 = blockIdx.x * p.run_units, u1 = min(u0 + p.run_units, p.total_units);
+  auto row_tile = [&](int t) { return p.rows_inner ? t % p.inner : t / p.inner; };
+  auto act_tile = [&](int t) { return p.rows_inner ? t / p.inner : t % p.inner; };
   const bool two_acc = p.mt <= 128;   // two accumulators: a tile's epilogue overlaps the next tile's products
   int* status = p.counters + kStatusIndex;
   bool dead = false;
@@ -220,8 +223,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
     // scale / zero of a unit's two stages: a row-strided (one line per thread) read that often comes from DRAM, so the
     // next unit's values are requested a whole unit before they are needed.  Position of the next request, kept by
     // counting: the divisions that derive it from the unit's number cost a third of a unit's dequantization.
-    int mt = u0 / ku, mk = u0 - mt * ku, mw = mt / p.mtiles, mm = mt - mw * p.mtiles, mg = 2 * mk / spg, mr = 2 * mk - mg * spg;
-    size_t mrow = (size_t)min(mw * kRows + r, p.N - 1) * p.ngroups;
+    int mt = u0 / ku, mk = u0 - mt * ku, m_out = mt / p.inner, m_in = mt - m_out * p.inner, mg = 2 * mk / spg, mr = 2 * mk - mg * spg;
+    size_t mrow = (size_t)min((p.rows_inner ? m_in : m_out) * kRows + r, p.N - 1) * p.ngroups;
     auto load_meta = [&] {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -231,8 +234,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
       }
       if (++mk == ku) {
         mk = mg = mr = 0;
-        if (++mm == p.mtiles) mm = 0, ++mw;
-        mrow = (size_t)min(mw * kRows + r, p.N - 1) * p.ngroups;
+        if (++m_in == p.inner) m_in = 0, ++m_out;
+        mrow = (size_t)min((p.rows_inner ? m_in : m_out) * kRows + r, p.N - 1) * p.ngroups;
       }
     };
     load_meta();
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
         const int t = u / ku, k = u - t * ku;
         bar_wait(raw_empty + slot * 8, par, status, dead);
         bar_expect(raw_full + slot * 8, kRawBytes);
-        tma_tile(raw + slot * kRawBytes, &tm_w, k * (kUnitK / 2), (t / p.mtiles) * kRows, raw_full + slot * 8);
+        tma_tile(raw + slot * kRawBytes, &tm_w, k * (kUnitK / 2), row_tile(t) * kRows, raw_full + slot * 8);
         if (++slot == rstages) slot = 0, par ^= 1;
       }
     }
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
       int s = 0;
       uint32_t par = 1;
       for (int u = u0; u < u1; ++u) {
-        const int t = u / ku, k = u - t * ku, m0 = (t % p.mtiles) * p.mt;
+        const int t = u / ku, k = u - t * ku, m0 = act_tile(t) * p.mt;
         for (int j = 0; j < 2; ++j) {
           bar_wait(ab_empty + s * 8, par, status, dead);
           bar_expect(ab_full + s * 8, b_stage);
@@ -346,7 +349,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
     for (int u = u0; u < u1; ++seg) {
       const int t = u / ku, k0 = u - t * ku, len = min(ku - k0, u1 - u);
       u += len;
-      const int row0 = (t / p.mtiles) * kRows, m0 = (t % p.mtiles) * p.mt;
+      const int row0 = row_tile(t) * kRows, m0 = act_tile(t) * p.mt;
       const int n = row0 + q4 * 32 + lane, mrows = min(p.mt, p.M - m0);
       const int buf = two_acc ? (seg & 1) : 0;
       const uint32_t acc = tmem + buf * 128 + ((uint32_t)(q4 * 32) << 16);
@@ -484,6 +487,7 @@ constexpr int kRingBytes = kMaxSmem - 1024 - 512;
 struct GemmPlan {
   int mt, mtiles, mpad, tiles, ku, run, ctas, stages, raw_stages;
   bool split;   // some tile lies in more than one run
+  int rows_inner;
 };
 
 // Heights of the activation tiles (a multiple of 16, what the MMA's N takes, all tiles alike) and runs (a CTA's share in
@@ -536,6 +540,14 @@ GemmPlan gemm_plan(int M, int N, int K) {
   if (g.raw_stages > kMaxRaw) g.raw_stages = kMaxRaw;
   g.ctas = (int)(((int64_t)g.tiles * g.ku + g.run - 1) / g.run);
   g.split = g.run % g.ku != 0;
+  // Tile order.  Activation tiles inner: a CTA stays with its weight rows, codes are read once.  When runs cut tiles, the CTAs are
+  // at different depths of different activation tiles, and activations that do not fit L2 then come from DRAM over and over
+  // (4999 x 14336 for 4096 rows: 4.6 GB in 600 us); with the weight tiles inner, neighbouring CTAs walk the same activation
+  // tile together: 636 -> 531 us, 8192 x 28672 with 3000 / 4999 rows 1545 / 2879 -> 1252 / 2246 us.  Whole tiles per CTA keep step
+  // by themselves, smaller activations stay in L2 (28672 x 4096, 1531 rows: 293 us, 309 the other way), and codes larger than
+  // the activations would be the ones re-read (57344 x 8192, 1000 rows: 1052 / 1418 us).
+  const double act = 2.0 * M * K, codes = 0.5 * N * K;
+  g.rows_inner = g.split && act > 126e6 && codes < act;
   return g;
 }
 
@@ -617,7 +629,8 @@ int gemm_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   p.ngroups = K / G;
   p.group_size = G;
   p.mt = g.mt;
-  p.mtiles = g.mtiles;
+  p.rows_inner = g.rows_inner;
+  p.inner = g.rows_inner ? g.tiles / g.mtiles : g.mtiles;
   p.tile_units = g.ku;
   p.total_units = g.tiles * g.ku;
   p.run_units = g.run;

@@ -64,3 +64,10 @@ def test_odd_output_pitch(cuda_lib):
     out = torch.zeros(50, 385, device="cuda", dtype=torch.float16)
     w4a16_forward(x, layer.packed_weight, sc, ze, 128, bias=bias, out=out[:, :384])
     assert torch.equal(out[:, :384], want) and bool((out[:, 384] == 0).all())
+
+
+def test_weight_tiles_inner(cuda_lib):
+    """Activations larger than L2 whose runs cut tiles: weight tiles are the inner direction of the order."""
+    layer = synthetic_linear(1000, 28672, seed=7, device="cuda")
+    x = torch.randn(2300, 28672, device="cuda", generator=torch.Generator("cuda").manual_seed(5)).half()
+    _check(layer, x)
