@@ -160,8 +160,8 @@ class QuantizedLinear(nn.Module):
 
     def _forward_kernel(self, x: Tensor) -> Tensor:
         bufs = self._kernel_buffers()
-        dtype, flat = x.dtype, x.dim() == 2
-        x2d = x if flat and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
+        dtype, flat = x.dtype, x.dim() == 2 and x.shape[1] == self.in_features   # else the last reshape refuses what does not fit
+        x2d = x if flat else x.reshape(-1, self.in_features)
         if dtype is not torch.float16 and dtype is not torch.bfloat16:
             x2d = x2d.to(torch.float16)
         if x2d.stride(1) != 1:

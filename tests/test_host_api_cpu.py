@@ -223,6 +223,31 @@ def test_awq_gemm_layout_roundtrip():
         to_awq_gemm(QuantizedLinear.from_linear(nn.Linear(256, 64), QuantConfig(bits=4, scheme="rtn", granularity="per_channel")))
 
 
+def _stubbed_layer(monkeypatch, in_features=256, out_features=64):
+    """A layer whose kernel call is replaced by a record of what it was given (rows of zeros come back)."""
+    layer = QuantizedLinear.from_linear(nn.Linear(in_features, out_features, bias=False), QuantConfig(bits=4, scheme="rtn", group_size=128))
+    given = []
+
+    def kernel(x, packed, scale, zero, group_size, **kw):
+        given.append(x)
+        return x.new_zeros(x.shape[0], packed.shape[0])
+
+    monkeypatch.setattr("pare_b200.kernels.matmul_int4.w4a16_forward", kernel)
+    return layer, given
+
+
+@pytest.mark.parametrize("shape", [(4, 128), (2, 512), (128,), (2, 3, 128)])
+def test_kernel_path_refuses_inputs_of_another_width(shape, monkeypatch):
+    """Rows are never joined or split to fit: as in the eager branch, an input whose last dimension is not in_features raises."""
+    layer, _ = _stubbed_layer(monkeypatch)
+    with pytest.raises(RuntimeError):
+        layer._forward_kernel(torch.randn(*shape).half())
+    with pytest.raises(RuntimeError):
+        layer(torch.randn(*shape))
+    for good in ((256,), (5, 256), (1, 256), (2, 3, 256), (0, 256)):
+        assert layer._forward_kernel(torch.randn(*good).half()).shape == (*good[:-1], 64)
+
+
 # ---- cache schedule ----------------------------------------------------------------------------------
 
 def test_plan_update_matches_oracle_state_machine():
