@@ -161,7 +161,8 @@ class QuantizedLinear(nn.Module):
     def _forward_kernel(self, x: Tensor) -> Tensor:
         bufs = self._kernel_buffers()
         dtype, flat = x.dtype, x.dim() == 2 and x.shape[1] == self.in_features   # else the last reshape refuses what does not fit
-        x2d = x if flat else x.reshape(-1, self.in_features)
+        # reshape also gives a single row (a slice of padded or broadcast rows) a pitch of its own
+        x2d = x if flat and (x.stride(0) == self.in_features or x.shape[0] > 1) else x.reshape(-1, self.in_features)
         if dtype is not torch.float16 and dtype is not torch.bfloat16:
             x2d = x2d.to(torch.float16)
         if x2d.stride(1) != 1:

@@ -248,6 +248,18 @@ def test_kernel_path_refuses_inputs_of_another_width(shape, monkeypatch):
         assert layer._forward_kernel(torch.randn(*good).half()).shape == (*good[:-1], 64)
 
 
+def test_kernel_path_takes_a_row_of_any_pitch(monkeypatch):
+    """One row out of rows that are broadcast (pitch 0) or padded to an odd pitch reaches the kernel as an ordinary row; several
+    rows keep their pitch."""
+    layer, given = _stubbed_layer(monkeypatch)
+    wide = torch.randn(4, 257).half()
+    for x in (torch.randn(256).half().expand(5, 256)[:1], wide[1:2, :256]):
+        assert layer._forward_kernel(x).shape == (1, 64)
+        assert given[-1].stride() == (256, 1) and torch.equal(given[-1], x)
+    layer._forward_kernel(wide[:, :256])
+    assert given[-1].stride() == (257, 1)
+
+
 # ---- cache schedule ----------------------------------------------------------------------------------
 
 def test_plan_update_matches_oracle_state_machine():
