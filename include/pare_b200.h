@@ -84,9 +84,9 @@ size_t pare_w4a16_workspace_bytes(int M, int N, int K, int group_size);
  * with whatever it has, and the call's result is then undefined.  pare_workspace_status synchronises `stream`,
  * returns the word (PARE_OK or PARE_ERR_TIMEOUT) and clears it; the word is sticky until read.  The same word
  * serves every entry point that takes this workspace (linear layers and decode attention).
- * pare_selftest_bounded_wait launches one thread that waits, through the kernels' own wait routine, at most
- * `polls` (<= 4096) polls on a shared-memory barrier that nothing arrives at, so the time-out path and this
- * accessor can be checked without a stuck kernel. */
+ * pare_selftest_bounded_wait waits, through the kernels' own wait routines, at most `polls` (<= 4096) polls (the
+ * tensor-memory kernels' routine: 100 ns each) on shared-memory barriers that nothing arrives at, so the time-out
+ * path and this accessor can be checked without a stuck kernel. */
 int pare_workspace_status(void* workspace, void* stream);
 int pare_selftest_bounded_wait(void* workspace, unsigned int polls, void* stream);
 
@@ -268,6 +268,12 @@ int pare_prefill_attn(const void* q, const void* k, const void* v, void* out, in
                       int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_t,
                       int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_t,
                       int B, int Hq, int H, int Tq, int Tk, int D, float softmax_scale, int causal, void* stream);
+
+/* Prompt attention has no workspace and so no status word: rows of a call in which a wait ran out are NaN.  This runs
+ * its tensor-memory kernel (causal, float16, dense [B][heads][T][128]) so that only `loads` tiles of keys and values
+ * ever arrive in a thread block and waits give up after `wait_us` (<= 10000) microseconds. */
+int pare_selftest_prefill_wait(const void* q, const void* k, const void* v, void* out, int B, int Hq, int H, int T,
+                               int loads, unsigned int wait_us, void* stream);
 
 /* ------------------------------------------------------------------------
  * Decode-step glue (no counterpart in the reference library: model code around the two hot

@@ -1,6 +1,7 @@
 // extern "C" surface of libpare_b200: argument checks and dispatch only.
 #include "peer.cuh"
 #include "prep.cuh"
+#include "tcgen05.cuh"
 
 namespace pare {
 struct ProducerArgs {
@@ -30,14 +31,32 @@ int gemm_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
 
 namespace pare {
 namespace {
-// A wait that nothing ends: one thread waits on a shared-memory barrier nobody arrives at, through the same bounded
-// wait the kernels use, with a caller-chosen (small) limit.  It returns after `limit` polls with the time-out recorded.
+// Waits that nothing ends, through the bounded waits the kernels use, with a caller-chosen (small) limit: one thread on a barrier
+// nobody arrives at (the streaming kernels' wait, limit in polls), then one warp on another (the tensor-memory kernels' wait,
+// limit in nanoseconds) which says so in a word of shared memory before it arrives where the second warp waits.  The word of the
+// workspace ends as the time-out only if the first wait recorded it and the second warp saw the other's.
 __global__ void bounded_wait_selftest_kernel(int* status, uint32_t limit) {
-  __shared__ uint64_t bar;
+  __shared__ uint64_t bars[3];
+  __shared__ int s_failed;
+  const uint32_t bar = gemv::smem_u32(bars);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  bool dead = false;
   if (threadIdx.x == 0) {
-    gemv::mbar_init(gemv::smem_u32(&bar), 1);
+    s_failed = 0;
+    for (int i = 0; i < 3; ++i) gemv::mbar_init(bar + i * 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    gemv::mbar_wait_limit(gemv::smem_u32(&bar), 0, status, limit);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) gemv::mbar_wait_limit(bar, 0, status, limit);
+  __syncthreads();
+  if (warp == 0) {
+    tc::bar_wait(bar + 8, 0, &s_failed, dead, 100ull * limit);
+    __syncwarp();
+    if (lane == 0) tc::bar_arrive(bar + 16);
+  } else {
+    tc::bar_wait(bar + 16, 0, &s_failed, dead);
+    const bool seen = *const_cast<volatile int*>(&s_failed) == PARE_ERR_TIMEOUT;
+    if (!__all_sync(0xffffffffu, seen && !dead) && lane == 0) atomicExch(status, PARE_ERR_CUDA);
   }
 }
 
@@ -252,7 +271,7 @@ int pare_workspace_status(void* workspace, void* stream) {
 int pare_selftest_bounded_wait(void* workspace, unsigned int polls, void* stream) {
   PARE_REQUIRE(workspace, PARE_ERR_WORKSPACE);
   PARE_REQUIRE(polls > 0 && polls <= 4096, PARE_ERR_SHAPE);   // a short wait by construction
-  pare::bounded_wait_selftest_kernel<<<1, 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  pare::bounded_wait_selftest_kernel<<<1, 64, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<int*>(workspace) + pare::gemv::kStatusIndex, polls);
   return cudaGetLastError() == cudaSuccess ? PARE_OK : PARE_ERR_CUDA;
 }

@@ -12,6 +12,8 @@
 // memory in 64-key tiles, two buffers, cp.async; S = Q K^T and O += P V on warp-level tensor-core steps
 // (m16n8k16, fp32 accumulate) with ldmatrix operand loads; softmax statistics online in registers, so the
 // score matrix never exists.  head_dim 128.
+#include <limits.h>
+
 #include "tcgen05.cuh"
 
 namespace pare {
@@ -267,6 +269,8 @@ struct TcParams {
   int ranks;           // work items per (batch, KV head), longest first
   float scale_log2;
   int causal;
+  int loads;           // K and V tiles that a CTA loads at most: all, except in the self test, where the rest never comes
+  uint64_t wait_ns;    // after which a wait gives up
 };
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -279,10 +283,14 @@ template <typename T>
 __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                                                                       const __grid_constant__ CUtensorMap tm_v, const TcParams p) {
   extern __shared__ unsigned char smem_dyn[];
+  // There is no status word on this path, so a wait that ran out must show in the result: the warp that gave up says so here and
+  // stops (nothing that follows from its data is committed or arrived at, so the others run out as well), and rows that
+  // are stored after that are NaN.  The CTA ends when its copies and products in flight have ended.
+  __shared__ int s_failed;
   const uint32_t base = (tc::s_u32(smem_dyn) + 1023u) & ~1023u;
   const uint32_t q_s = base, ring = base + 2 * kTTile, bars = ring + kTRing * kTTile;
   const uint32_t q_full = bars, kv_full = bars + 8, kv_empty = kv_full + kTRing * 8, s_full = kv_empty + kTRing * 8, p_full = s_full + 16,
-                 tmem_slot = p_full + 16;
+                 mma_done = p_full + 16, tmem_slot = mma_done + 8;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform, and known to be
   bool dead = false;
 
@@ -319,7 +327,9 @@ __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __g
   const int nk0 = tiles_of(qt0), nk1 = tiles_of(qt1);   // nk0 >= nk1
 
   if (threadIdx.x == 0) {
+    s_failed = 0;
     tc::bar_init(q_full, 1);
+    tc::bar_init(mma_done, 1);
     for (int i = 0; i < kTRing; ++i) {
       tc::bar_init(kv_full + i * 8, 1);
       tc::bar_init(kv_empty + i * 8, 1);
@@ -352,16 +362,20 @@ __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __g
         tc::tma_tile4(q_s + kTTile, &tm_q, 0, qt1 * kTQ, hq1, b, q_full);
         tc::tma_tile4(q_s + kTTile + kTTile / 2, &tm_q, 64, qt1 * kTQ, hq1, b, q_full);
       }
-      int slot = 0;
+      int slot = 0, i = 0;
       uint32_t par = 1;
-      for (int i = 0; i < 2 * nk0; ++i) {
-        tc::bar_wait(kv_empty + slot * 8, par, nullptr, dead);
+      for (const int n = min(2 * nk0, p.loads); i < n; ++i) {
+        tc::bar_wait(kv_empty + slot * 8, par, &s_failed, dead, p.wait_ns);
+        if (dead) break;
         tc::bar_expect(kv_full + slot * 8, kTTile);
         const CUtensorMap* map = (i & 1) ? &tm_v : &tm_k;
         tc::tma_tile4(ring + slot * kTTile, map, 0, (i >> 1) * kTK, h, b, kv_full + slot * 8);
         tc::tma_tile4(ring + slot * kTTile + kTTile / 2, map, 64, (i >> 1) * kTK, h, b, kv_full + slot * 8);
         if (++slot == kTRing) slot = 0, par ^= 1;
       }
+      bool late = false;
+      tc::bar_wait(q_full, 0, &s_failed, late);
+      for (int j = max(0, i - kTRing); j < i; ++j) tc::bar_wait(kv_full + (j % kTRing) * 8, (j / kTRing) & 1, &s_failed, late);
     }
     __syncwarp();
   } else if (warp == 9) {
@@ -390,40 +404,46 @@ __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __g
       };
       int slot = 0;
       uint32_t par = 0;
+      auto wait = [&](uint32_t bar, uint32_t parity) {   // for the whole warp; dead if a lane gave up
+        tc::bar_wait(bar, parity, &s_failed, dead, p.wait_ns);
+        dead = __any_sync(0xffffffffu, dead);
+      };
       auto take = [&](uint32_t& bar_empty) {   // next tile of the ring, in load order
-        tc::bar_wait(kv_full + slot * 8, par, nullptr, dead);
-        __syncwarp();
+        wait(kv_full + slot * 8, par);
         const uint32_t addr = ring + slot * kTTile;
         bar_empty = kv_empty + slot * 8;
         if (++slot == kTRing) slot = 0, par ^= 1;
         return addr;
       };
-      tc::bar_wait(q_full, 0, nullptr, dead);
+      wait(q_full, 0);
       uint32_t k_empty, v_empty;
       uint32_t ks = take(k_empty);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      qk(0, ks);
-      tc::umma_commit(s_full, me);
-      if (nk1 > 0) {
-        qk(1, ks);
-        tc::umma_commit(s_full + 8, me);
+      if (!dead) {
+        qk(0, ks);
+        tc::umma_commit(s_full, me);
+        if (nk1 > 0) {
+          qk(1, ks);
+          tc::umma_commit(s_full + 8, me);
+        }
+        tc::umma_commit(k_empty, me);
       }
-      tc::umma_commit(k_empty, me);
       for (int t = 0; t < nk0; ++t) {
         const uint32_t vs = take(v_empty);
         const bool more = t + 1 < nk0;
-        tc::bar_wait(p_full, t & 1, nullptr, dead);
-        __syncwarp();
+        wait(p_full, t & 1);
+        if (dead) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         pv(0, vs, t == 0);
         if (more) {
           ks = take(k_empty);
+          if (dead) break;
           qk(0, ks);
         }
         tc::umma_commit(s_full, me);       // S of the next tile (or, after the last, O) is complete -- and with it P V so far
         if (t < nk1) {
-          tc::bar_wait(p_full + 8, t & 1, nullptr, dead);
-          __syncwarp();
+          wait(p_full + 8, t & 1);
+          if (dead) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           pv(1, vs, t == 0);
           if (t + 1 < nk1) qk(1, ks);
@@ -432,6 +452,9 @@ __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __g
         tc::umma_commit(v_empty, me);
         if (more) tc::umma_commit(k_empty, me);
       }
+      tc::umma_commit(mma_done, me);
+      bool late = false;
+      tc::bar_wait(mma_done, 0, &s_failed, late);
     }
     __syncwarp();
   } else {
@@ -445,8 +468,9 @@ __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __g
     float m_ref = 0.f, l = 0.f;
     bool seen = false;   // m_ref is the scaled maximum of something visible
     for (int t = 0; t < nk; ++t) {
-      tc::bar_wait(s_full + half * 8, t & 1, nullptr, dead);
-      __syncwarp();
+      tc::bar_wait(s_full + half * 8, t & 1, &s_failed, dead, p.wait_ns);
+      dead = __any_sync(0xffffffffu, dead);
+      if (dead) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int key0 = t * kTK;
       const bool mask = __any_sync(0xffffffffu, key0 + kTK - 1 > key_lim);
@@ -529,10 +553,9 @@ __global__ void __launch_bounds__(kTThreads, 1) prefill_attn_tc_kernel(const __g
       if (lane == 0) tc::bar_arrive(p_full + half * 8);
     }
     if (nk > 0) {
-      tc::bar_wait(s_full + half * 8, nk & 1, nullptr, dead);
-      dead = __any_sync(0xffffffffu, dead);
+      tc::bar_wait(s_full + half * 8, nk & 1, &s_failed, dead, p.wait_ns);
+      dead = __any_sync(0xffffffffu, dead || *const_cast<volatile int*>(&s_failed) != 0);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // a wait that ran out (there is no status word on this path) must not pass for a result
       const float inv = dead ? __int_as_float(0x7fffffff) : (l > 0.f ? 1.f / l : (l == 0.f ? 0.f : l));
       T* og = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_sb + (int64_t)hq * p.o_sh + (int64_t)row * p.o_st;
 #pragma unroll 1
@@ -584,8 +607,50 @@ bool tc_map(CUtensorMap* map, const void* base, int dtype, int64_t sb, int64_t s
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The tensor-memory kernel; PARE_ERR_UNSUPPORTED where no tensor map describes the operands.
+int prefill_tc(const PrefillParams& p, int dtype, int loads, uint64_t wait_ns, cudaStream_t s) {
+  TcParams tp{};
+  tp.out = p.out; tp.o_sb = p.o_sb; tp.o_sh = p.o_sh; tp.o_st = p.o_st;
+  tp.H = p.H; tp.rep = p.rep; tp.Tq = p.Tq; tp.Tk = p.Tk;
+  tp.n_qt = (p.Tq + kTQ - 1) / kTQ;
+  tp.ranks = (p.rep & 1) ? tp.n_qt / 2 * p.rep + (tp.n_qt & 1) * ((p.rep + 1) / 2) : tp.n_qt * (p.rep / 2);
+  tp.scale_log2 = p.scale_log2;
+  tp.causal = p.causal;
+  tp.loads = loads;
+  tp.wait_ns = wait_ns;
+  CUtensorMap mq, mk, mv;
+  const int64_t ctas = (int64_t)tp.ranks * p.H * p.B;
+  if (ctas >= ((int64_t)1 << 31) || !tc_map(&mq, p.q, dtype, p.q_sb, p.q_sh, p.q_st, p.B, p.Hq, p.Tq) ||
+      !tc_map(&mk, p.k, dtype, p.k_sb, p.k_sh, p.k_st, p.B, p.H, p.Tk) || !tc_map(&mv, p.v, dtype, p.v_sb, p.v_sh, p.v_st, p.B, p.H, p.Tk))
+    return PARE_ERR_UNSUPPORTED;
+  auto launch = [&](auto kern) -> int {
+    if (!ensure_smem_attr(reinterpret_cast<const void*>(kern), (int)kTSmem)) return PARE_ERR_CUDA;
+    kern<<<(unsigned)ctas, kTThreads, kTSmem, s>>>(mq, mk, mv, tp);
+    return launch_status();
+  };
+  return dtype == PARE_F16 ? launch(prefill_attn_tc_kernel<__half>) : launch(prefill_attn_tc_kernel<__nv_bfloat16>);
+}
+
 }  // namespace
 }  // namespace pare
+
+extern "C" int pare_selftest_prefill_wait(const void* q, const void* k, const void* v, void* out, int B, int Hq, int H, int T, int loads,
+                                          unsigned int wait_us, void* stream) {
+  using namespace pare;
+  PARE_REQUIRE(q && k && v && out && B > 0 && Hq > 0 && H > 0 && Hq % H == 0 && T > 0 && loads >= 0, PARE_ERR_SHAPE);
+  PARE_REQUIRE(wait_us <= 10000, PARE_ERR_SHAPE);   // short waits by construction
+  PARE_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out), PARE_ERR_ALIGN);
+  PrefillParams p{};
+  p.q = q; p.k = k; p.v = v; p.out = out;
+  p.q_st = p.k_st = p.v_st = p.o_st = kPD;
+  p.q_sh = p.k_sh = p.v_sh = p.o_sh = (int64_t)T * kPD;
+  p.q_sb = p.o_sb = p.q_sh * Hq;
+  p.k_sb = p.v_sb = p.k_sh * H;
+  p.B = B; p.Hq = Hq; p.H = H; p.rep = Hq / H; p.Tq = p.Tk = T;
+  p.scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
+  p.causal = 1;
+  return prefill_tc(p, PARE_F16, loads, 1000ull * wait_us, reinterpret_cast<cudaStream_t>(stream));
+}
 
 extern "C" int pare_prefill_attn(const void* q, const void* k, const void* v, void* out, int dtype, int64_t q_stride_b,
                                  int64_t q_stride_h, int64_t q_stride_t, int64_t k_stride_b, int64_t k_stride_h,
@@ -617,24 +682,8 @@ extern "C" int pare_prefill_attn(const void* q, const void* k, const void* v, vo
   // 9.0 us there, 6.6 us here; 128 tokens 10.3 / 9.5; 4 x 200 tokens 13.1 / 32.0; 512 tokens 18.5 / 33.9; 8192 tokens
   // 640 / 3250).  The kernel above serves the rest.
   if (softmax_scale > 0.f && Tk > kPK) {
-    TcParams tp{};
-    tp.out = out; tp.o_sb = out_stride_b; tp.o_sh = out_stride_h; tp.o_st = out_stride_t;
-    tp.H = H; tp.rep = p.rep; tp.Tq = Tq; tp.Tk = Tk;
-    tp.n_qt = (Tq + kTQ - 1) / kTQ;
-    tp.ranks = (p.rep & 1) ? tp.n_qt / 2 * p.rep + (tp.n_qt & 1) * ((p.rep + 1) / 2) : tp.n_qt * (p.rep / 2);
-    tp.scale_log2 = p.scale_log2;
-    tp.causal = p.causal;
-    CUtensorMap mq, mk, mv;
-    const int64_t ctas = (int64_t)tp.ranks * H * B;
-    if (ctas < ((int64_t)1 << 31) && tc_map(&mq, q, dtype, q_stride_b, q_stride_h, q_stride_t, B, Hq, Tq) &&
-        tc_map(&mk, k, dtype, k_stride_b, k_stride_h, k_stride_t, B, H, Tk) && tc_map(&mv, v, dtype, v_stride_b, v_stride_h, v_stride_t, B, H, Tk)) {
-      auto launch = [&](auto kern) -> int {
-        if (!ensure_smem_attr(reinterpret_cast<const void*>(kern), (int)kTSmem)) return PARE_ERR_CUDA;
-        kern<<<(unsigned)ctas, kTThreads, kTSmem, s>>>(mq, mk, mv, tp);
-        return launch_status();
-      };
-      return dtype == PARE_F16 ? launch(prefill_attn_tc_kernel<__half>) : launch(prefill_attn_tc_kernel<__nv_bfloat16>);
-    }
+    const int rc = prefill_tc(p, dtype, INT_MAX, tc::kWaitNs, s);
+    if (rc != PARE_ERR_UNSUPPORTED) return rc;
   }
   const dim3 grid((Tq + kPQ - 1) / kPQ, Hq, B);
   auto launch = [&](auto kern) -> int {

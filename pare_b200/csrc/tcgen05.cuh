@@ -33,8 +33,9 @@ __device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: two seconds of the global timer.  `dead` is sticky per thread: after one expiry nothing waits any more.
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, int* status, bool& dead) {
+// Bounded wait: `limit_ns` of the global timer.  `dead` is sticky per thread: after one expiry nothing waits any more.  `status`
+// (global, or shared by the CTA) is set before this returns, so whoever sees an arrival that follows sees it too.
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, int* status, bool& dead, uint64_t limit_ns = kWaitNs) {
   if (dead || bar_test(bar, parity)) return;
   uint64_t t0 = 0, t1 = 0;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
@@ -44,9 +45,10 @@ __device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, int* sta
     for (int i = 0; i < kPolls; ++i)
       if (bar_test(bar, parity)) return;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-  } while (t1 - t0 < kWaitNs);
+  } while (t1 - t0 < limit_ns);
   dead = true;
-  if (status) atomicExch(status, PARE_ERR_TIMEOUT);
+  atomicExch(status, PARE_ERR_TIMEOUT);
+  __threadfence_block();
 }
 __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(

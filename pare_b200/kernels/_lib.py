@@ -57,6 +57,7 @@ SIGNATURES: dict[str, tuple] = {
                                    _i, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pare_prefill_attn": (_i, [_vp, _vp, _vp, _vp, _i, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
                                _i, _i, _i, _i, _i, _i, C.c_float, _i, _vp]),
+    "pare_selftest_prefill_wait": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, C.c_uint, _vp]),
     "pare_rmsnorm_residual": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, C.c_float, _i, _vp]),
     "pare_silu_mul": (_i, [_vp, _vp, _vp, _i, _i, _i64, _i, _vp]),
     "pare_rope": (_i, [_vp, _i64, _i64, _i64, _vp, _vp, _i, _i, _i, _i, _i, _vp]),

@@ -83,3 +83,22 @@ def test_infinite_logit_gives_nan_and_hidden_keys_do_not_matter(cuda_lib):
     k[0, 0, 64] = float("inf")
     out = prefill_attention(q, k, v)
     assert bool(torch.isfinite(out[:, :, :64]).all()) and bool(torch.isnan(out[:, :, 64:]).all())
+
+
+@pytest.mark.parametrize("loads", [0, 1, 2, 3, 7])
+@pytest.mark.parametrize("hq,h,t", [(2, 1, 600), (3, 1, 600), (1, 1, 100)])
+def test_a_wait_that_runs_out_gives_nan(hq, h, t, loads, cuda_lib):
+    """Key and value tiles that never arrive: whichever warp gives up first, no row that depends on them passes for a result, and the
+    next call is served as ever.  (Query tiles that had all they need before that are as they should be.)"""
+    g = torch.Generator("cuda").manual_seed(loads)
+    q = torch.randn(1, hq, t, 128, device="cuda", generator=g).half()
+    k = torch.randn(1, h, t, 128, device="cuda", generator=g).half()
+    v = torch.randn(1, h, t, 128, device="cuda", generator=g).half()
+    want, out = prefill_attention(q, k, v), torch.zeros_like(q)
+    assert cuda_lib.pare_selftest_prefill_wait(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1, hq, h, t, loads, 300,
+                                               torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    whole = loads // 2 * 128                       # keys whose K and V tiles both arrive
+    assert bool(torch.isnan(out[:, :, whole:]).all())
+    assert bool((torch.isnan(out[:, :, :whole]) | (out[:, :, :whole] == want[:, :, :whole])).all())
+    assert torch.equal(prefill_attention(q, k, v), want)
