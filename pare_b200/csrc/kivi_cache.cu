@@ -646,6 +646,7 @@ int pare_kivi_dense(const uint8_t* k_codes, const float* k_scale, const float* k
   PARE_REQUIRE(out_k && out_v && n_comp >= 0 && n_comp <= cap && n_comp % group == 0 && n_res >= 0 && n_new >= 0, PARE_ERR_SHAPE);
   PARE_REQUIRE(n_res + n_new == 0 || (res_k && res_v), PARE_ERR_SHAPE);
   PARE_REQUIRE(n_new == 0 || (new_k && new_v), PARE_ERR_SHAPE);
+  PARE_REQUIRE(B <= 65535 && H <= 65535, PARE_ERR_UNSUPPORTED);   // the launch grid
   if (n_comp + n_res + n_new == 0) return PARE_OK;
   const size_t esz = dtype == PARE_F32 ? 4 : 2;
   for (int64_t st : {res_stride_b, res_stride_h, res_stride_t, new_k_stride_b, new_k_stride_h, new_k_stride_t, new_v_stride_b,

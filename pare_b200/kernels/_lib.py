@@ -117,6 +117,11 @@ def dtype_code(dtype: torch.dtype) -> int:
         raise KernelLibraryError(f"dtype {dtype} is not supported by libpare_b200") from None
 
 
+def has_code(dtype: torch.dtype) -> bool:
+    """True for the dtypes the kernels take."""
+    return dtype in _DTYPE_CODE
+
+
 def check(status: int, what: str) -> None:
     if status != 0:
         msg = lib().pare_status_string(status).decode()

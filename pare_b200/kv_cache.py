@@ -347,20 +347,40 @@ class QuantizedKVCache:
         """Append ``[B, H, new_tokens, D]`` keys / values; return the dense ``(K, V)`` of the whole
         sequence in the input dtype (reference contract, ``pare/kv_cache.py:205-252``)."""
         st, left_k, left_v = self._append(layer_idx, new_k, new_v, defer_window=True)
+        try:
+            return self._dense(st, left_k, left_v)
+        except BaseException:
+            # the new tokens are counted already: whatever failed (the dense result is the largest allocation of a step), they
+            # have to be in the window
+            self._store_left(st, left_k, left_v)
+            raise
+
+    @staticmethod
+    def _store_left(st: _LayerStore, left_k: Tensor | None, left_v: Tensor | None) -> None:
+        """Copy tokens that ``_append`` left to its caller to the end of the window."""
+        if left_k is not None:
+            st.res_k[:, :, st.r_len - left_k.shape[2]: st.r_len] = left_k
+            st.res_v[:, :, st.r_len - left_v.shape[2]: st.r_len] = left_v
+
+    def _dense(self, st: _LayerStore, left_k: Tensor | None, left_v: Tensor | None) -> tuple[Tensor, Tensor]:
+        """Dense ``(K, V)`` of everything in the store; ``left_k / left_v`` (the newest tokens of the window, or ``None``) are
+        stored in the window on the way."""
         total = st.n_comp + st.r_len
         full_k = torch.empty(st.B, st.H, total, st.D, device=st.device, dtype=st.dtype)
         full_v = torch.empty_like(full_k)
-        if total == 0:
+        if full_k.numel() == 0:
             return full_k, full_v
         n_left = 0 if left_k is None else left_k.shape[2]
         n_old = st.r_len - n_left
-        code, stream = _lib.dtype_code(st.dtype), _lib.current_stream(st.device)
+        stream = _lib.current_stream(st.device)
         status = _lib.UNSUPPORTED
-        # one launch: reconstructed tokens, window, and the tokens that are on their way into the window
-        if not (st.res_k.requires_grad or st.res_v.requires_grad):
+        # One launch: reconstructed tokens, window, and the tokens that are on their way into the window.  Tokens that only ever were
+        # copied (dtypes without a kernel, a store on another device than the current one) still are.
+        if (_lib.has_code(st.dtype) and not (st.res_k.requires_grad or st.res_v.requires_grad)
+                and torch.cuda.current_device() == st.device.index):
             status = _lib.lib().pare_kivi_dense(
                 *st.cache_args(), *st.geometry(), st.n_comp,
-                full_k.data_ptr(), full_v.data_ptr(), code, full_k.stride(0), full_k.stride(1), full_k.stride(2),
+                full_k.data_ptr(), full_v.data_ptr(), _lib.dtype_code(st.dtype), full_k.stride(0), full_k.stride(1), full_k.stride(2),
                 st.res_k.data_ptr(), st.res_v.data_ptr(), st.res_k.stride(0), st.res_k.stride(1), st.res_k.stride(2), n_old,
                 *((left_k.data_ptr(), left_v.data_ptr(), left_k.stride(0), left_k.stride(1), left_k.stride(2),
                    left_v.stride(0), left_v.stride(1), left_v.stride(2)) if n_left else (None, None, 0, 0, 0, 0, 0, 0)),
@@ -369,13 +389,11 @@ class QuantizedKVCache:
             return full_k, full_v
         if status != _lib.UNSUPPORTED:
             _lib.check(status, "pare_kivi_dense")
-        if n_left:
-            st.res_k[:, :, n_old:st.r_len] = left_k
-            st.res_v[:, :, n_old:st.r_len] = left_v
+        self._store_left(st, left_k, left_v)
         if st.n_comp > 0:
             status = _lib.lib().pare_kivi_dequant(
                 *st.cache_args(), *st.geometry(), st.n_comp,
-                full_k.data_ptr(), full_v.data_ptr(), code,
+                full_k.data_ptr(), full_v.data_ptr(), _lib.dtype_code(st.dtype),
                 full_k.stride(0), full_k.stride(1), full_k.stride(2), stream,
             )
             _lib.check(status, "pare_kivi_dequant")

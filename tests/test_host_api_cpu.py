@@ -19,6 +19,7 @@ from pare_b200 import KVCacheConfig, QuantConfig, QuantDtype, QuantizedKVCache, 
 from pare_b200.core import compute_scale, dequantize_tensor, pack_int4, quantize_tensor, unpack_int4
 from pare_b200.core.pack import (pack_int4_signed, packed_size_bytes, repack_int4_for_kernel, unpack_int4_signed,
                                  unrepack_int4_from_kernel)
+from pare_b200 import kv_cache
 from pare_b200.kernels import _lib
 from pare_b200.kv_cache import plan_update
 
@@ -284,6 +285,70 @@ def test_cache_host_api_without_gpu():
     with pytest.raises(ValueError):
         QuantizedKVCache(1, KVCacheConfig(bits=3))
     cache.reset()
+
+
+class _CountingLib:
+    """Stands in for the CUDA library: every call is counted and answers with a given status (0 where none is given)."""
+
+    def __init__(self, **status):
+        self.status, self.calls = status, []
+
+    def __getattr__(self, name):
+        if name == "pare_status_string":
+            return lambda code: b"stub"
+
+        def call(*args):
+            self.calls.append(name)
+            return self.status.get(name, 0)
+        return call
+
+
+def _stubbed_cache(monkeypatch, lib, shape=(1, 2, 128), dtype=torch.float16, **cfg):
+    cache = QuantizedKVCache(1, KVCacheConfig(bits=4, group_size=32, residual_length=64, **cfg))
+    cache._stores[0] = kv_cache._LayerStore(*shape, cache.config, 1024, torch.device("cpu"), dtype)
+    for t in (cache._stores[0].res_k, cache._stores[0].res_v):
+        t.fill_(-77.0)
+    monkeypatch.setattr(_lib, "lib", lambda: lib)
+    monkeypatch.setattr(_lib, "current_stream", lambda device: 0)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: None)      # the index of the stub store's device
+    return cache
+
+
+@pytest.mark.parametrize("n", [1, 40, 500])
+@pytest.mark.parametrize("failure", ["allocation", "launch"])
+def test_update_that_fails_keeps_the_tokens(n, failure, monkeypatch):
+    """The dense result cannot be allocated, or its launch fails: the tokens that count as appended are in the window."""
+    lib = _CountingLib(pare_kivi_dense=6)
+    cache = _stubbed_cache(monkeypatch, lib)
+    k, v = torch.randn(1, 2, n, 128).half(), torch.randn(1, 2, n, 128).half()
+    if failure == "allocation":
+        def no_memory(*a, **kw):
+            raise torch.cuda.OutOfMemoryError("no memory")
+        monkeypatch.setattr(torch, "empty", no_memory)
+    with pytest.raises(RuntimeError):
+        cache.update(0, k, v)
+    monkeypatch.undo()
+    held = cache._residual_k[0].shape[2]
+    assert cache.seq_len(0) == n and 0 < held <= n
+    assert torch.equal(cache._residual_k[0], k[:, :, -held:]) and torch.equal(cache._residual_v[0], v[:, :, -held:])
+
+
+def test_update_of_what_no_kernel_takes(monkeypatch):
+    """Tokens that fit the window and were only ever copied: float64, no sequences at all, a store that is not on the current device."""
+    k, v = torch.randn(1, 2, 9, 128), torch.randn(1, 2, 9, 128)
+    cache = _stubbed_cache(monkeypatch, _CountingLib(pare_kivi_dense=2), dtype=torch.float64)
+    got = cache.update(0, k.double(), v.double())
+    assert torch.equal(got[0], k.double()) and torch.equal(got[1], v.double()) and cache.seq_len(0) == 9
+
+    cache = _stubbed_cache(monkeypatch, _CountingLib(pare_kivi_dense=1), shape=(0, 2, 128))
+    got = cache.update(0, k[:0].half(), v[:0].half())
+    assert got[0].shape == got[1].shape == (0, 2, 9, 128) and cache.seq_len(0) == 9
+
+    lib = _CountingLib()
+    cache = _stubbed_cache(monkeypatch, lib)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    got = cache.update(0, k.half(), v.half())
+    assert torch.equal(got[0], k.half()) and torch.equal(got[1], v.half()) and lib.calls == []
 
 
 # ---- the C ABI ------------------------------------------------------------------------------------------
