@@ -30,6 +30,7 @@ from dataclasses import dataclass
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 
 from pare_b200.kernels import _lib
 
@@ -113,6 +114,13 @@ def plan_update(r_len: int, n_new: int, residual_length: int, group_size: int) -
     total = r_len + n_new
     n_c = (max(0, total - residual_length) // group_size) * group_size
     return n_c, total - n_c
+
+
+def _only_numbers(*tensors: Tensor) -> bool:
+    """True if a kernel that reads or writes these tensors by address leaves nothing out that a copy would carry along: no gradient,
+    no tangent, no subclass with a behaviour of its own."""
+    return all(type(t) is Tensor and not (t.requires_grad and torch.is_grad_enabled())
+               and (forward_ad._current_level < 0 or forward_ad.unpack_dual(t).tangent is None) for t in tensors)
 
 
 def _roundup(x: int, m: int) -> int:
@@ -292,10 +300,11 @@ class QuantizedKVCache:
         if rope is not None and not deferred:   # the kernel rotates only a key it appends itself
             new_k = apply_rope(new_k, rope)
         left_k = left_v = None   # with defer_window: what the caller copies into the window
-        # kernels may read the new tokens where they are: same device and dtype as the store, nothing for autograd to see
+        # kernels may read the new tokens where they are: same device and dtype as the store, nothing for autograd to see (the
+        # tokens before them may have left something in the window)
         plain = not deferred and (new_k.device == st.device and new_v.device == st.device and new_v.dtype == st.dtype
                                   and new_k.stride(3) == 1 and new_v.stride(3) == 1
-                                  and not (torch.is_grad_enabled() and (new_k.requires_grad or new_v.requires_grad)))
+                                  and _only_numbers(new_k, new_v))
         from_empty = plain and st.r_len == 0
         if deferred:
             pass
@@ -376,7 +385,7 @@ class QuantizedKVCache:
         status = _lib.UNSUPPORTED
         # One launch: reconstructed tokens, window, and the tokens that are on their way into the window.  Tokens that only ever were
         # copied (dtypes without a kernel, a store on another device than the current one) still are.
-        if (_lib.has_code(st.dtype) and not (st.res_k.requires_grad or st.res_v.requires_grad)
+        if (_lib.has_code(st.dtype) and not (st.res_k.requires_grad or st.res_v.requires_grad) and _only_numbers(st.res_k, st.res_v)
                 and torch.cuda.current_device() == st.device.index):
             status = _lib.lib().pare_kivi_dense(
                 *st.cache_args(), *st.geometry(), st.n_comp,

@@ -351,6 +351,27 @@ def test_update_of_what_no_kernel_takes(monkeypatch):
     assert torch.equal(got[0], k.half()) and torch.equal(got[1], v.half()) and lib.calls == []
 
 
+class _Tagged(torch.Tensor):
+    """A tensor subclass: what is done to it goes through the dispatcher."""
+
+
+def test_update_carries_what_a_copy_would(monkeypatch):
+    """Tokens with a tangent (forward-mode differentiation), now or earlier in the window, and tensor subclasses are copied by torch."""
+    k, v = torch.randn(1, 2, 9, 128).half(), torch.randn(1, 2, 9, 128).half()
+    tangent = torch.randn(1, 2, 9, 128).half()
+    lib = _CountingLib()
+    cache = _stubbed_cache(monkeypatch, lib)
+    with torch.autograd.forward_ad.dual_level():
+        got, _ = cache.update(0, torch.autograd.forward_ad.make_dual(k, tangent), v)
+        later, _ = cache.update(0, k[:, :, :1], v[:, :, :1])
+        assert torch.equal(torch.autograd.forward_ad.unpack_dual(got).tangent, tangent)
+        assert torch.equal(torch.autograd.forward_ad.unpack_dual(later).tangent[:, :, :9], tangent)
+    assert lib.calls == []
+    cache = _stubbed_cache(monkeypatch, lib)
+    left = cache._append(0, k.as_subclass(_Tagged), v, defer_window=True)
+    assert left[1] is None and torch.equal(cache._residual_k[0], k) and lib.calls == []
+
+
 # ---- the C ABI ------------------------------------------------------------------------------------------
 
 def test_library_exports_every_declared_symbol():
