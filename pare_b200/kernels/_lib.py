@@ -152,6 +152,10 @@ def w4a16_workspace_bytes(m: int, n: int, k: int, group_size: int) -> int:
 
 # One zero-initialised workspace per device and stream; the kernels leave it zero-consistent.
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
+# Workspaces that were too small for a later call.  A CUDA graph captured before that call still works in them, whoever captured it
+# (stream handles come from a pool and serve several owners), so they are not given back; each is at most half as large as the
+# next of its stream, so together they stay smaller than the one in use.
+_outgrown: list[torch.Tensor] = []
 
 
 def workspace_status(device: torch.device) -> int:
@@ -170,7 +174,9 @@ def workspace(device: torch.device, nbytes: int, stream: int | None = None) -> t
     key = (_index(device), current_stream(device) if stream is None else stream)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
-        size = max(nbytes, 8 << 20)
-        buf = torch.zeros(size, dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
+        size = max(nbytes, 8 << 20 if buf is None else 2 * buf.numel())
+        larger = torch.zeros(size, dtype=torch.uint8, device=device)
+        if buf is not None:
+            _outgrown.append(buf)
+        _workspaces[key] = buf = larger
     return buf

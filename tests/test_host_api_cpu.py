@@ -5,6 +5,7 @@ tests/test_triton_kernel.py:42-101, tests/test_model_io.py.)"""
 
 import ctypes
 import re
+import weakref
 from pathlib import Path
 
 import numpy as np
@@ -370,6 +371,26 @@ def test_update_carries_what_a_copy_would(monkeypatch):
     cache = _stubbed_cache(monkeypatch, lib)
     left = cache._append(0, k.as_subclass(_Tagged), v, defer_window=True)
     assert left[1] is None and torch.equal(cache._residual_k[0], k) and lib.calls == []
+
+
+# ---- workspaces ---------------------------------------------------------------------------------------
+
+def test_outgrown_workspaces_stay_where_they_are(monkeypatch):
+    """A graph captured with a stream's workspace works in it at every replay: growing the workspace must not free it.  What is kept
+    stays smaller than what is in use."""
+    monkeypatch.setattr(_lib, "_workspaces", {})
+    monkeypatch.setattr(_lib, "_outgrown", [], raising=False)
+    monkeypatch.setattr(_lib, "_index", lambda device: 0)
+    cpu = torch.device("cpu")
+    alive = []
+    for nbytes in (1 << 20, 8 << 20, (8 << 20) + 1, 18 << 20, 100 << 20):
+        buf = _lib.workspace(cpu, nbytes, 7)
+        assert buf.numel() >= nbytes and not buf.any()
+        alive.append(weakref.ref(buf))
+        del buf
+    assert all(ref() is not None for ref in alive) and len({id(ref()) for ref in alive}) == 4
+    assert sum(b.numel() for b in _lib._outgrown) < _lib.workspace(cpu, 1, 7).numel()
+    assert _lib.workspace(cpu, 1, 8).numel() == 8 << 20
 
 
 # ---- the C ABI ------------------------------------------------------------------------------------------
