@@ -138,6 +138,11 @@ def _index(device: torch.device) -> int:
     return torch.cuda.current_device() if index is None else index
 
 
+def current_device() -> int:
+    """Index of the current CUDA device (``torch.cuda.current_device`` once CUDA is in use)."""
+    return torch._C._cuda_getDevice()
+
+
 def current_stream(device: torch.device) -> int:
     """Handle of the current stream of ``device`` (the raw handle: a ``torch.cuda.Stream`` object per launch costs more
     than some of the launches)."""

@@ -116,11 +116,11 @@ def plan_update(r_len: int, n_new: int, residual_length: int, group_size: int) -
     return n_c, total - n_c
 
 
-def _only_numbers(*tensors: Tensor) -> bool:
-    """True if a kernel that reads or writes these tensors by address leaves nothing out that a copy would carry along: no gradient,
+def _only_numbers(a: Tensor, b: Tensor) -> bool:
+    """True if a kernel that reads or writes the two tensors by address leaves nothing out that a copy would carry along: no gradient,
     no tangent, no subclass with a behaviour of its own."""
-    return all(type(t) is Tensor and not (t.requires_grad and torch.is_grad_enabled())
-               and (forward_ad._current_level < 0 or forward_ad.unpack_dual(t).tangent is None) for t in tensors)
+    return (type(a) is Tensor and type(b) is Tensor and not ((a.requires_grad or b.requires_grad) and torch.is_grad_enabled())
+            and (forward_ad._current_level < 0 or (forward_ad.unpack_dual(a).tangent is None and forward_ad.unpack_dual(b).tangent is None)))
 
 
 def _roundup(x: int, m: int) -> int:
@@ -385,14 +385,15 @@ class QuantizedKVCache:
         status = _lib.UNSUPPORTED
         # One launch: reconstructed tokens, window, and the tokens that are on their way into the window.  Tokens that only ever were
         # copied (dtypes without a kernel, a store on another device than the current one) still are.
-        if (_lib.has_code(st.dtype) and not (st.res_k.requires_grad or st.res_v.requires_grad) and _only_numbers(st.res_k, st.res_v)
-                and torch.cuda.current_device() == st.device.index):
+        res_k, res_v = st.res_k, st.res_v
+        if (_lib.has_code(st.dtype) and not (res_k.requires_grad or res_v.requires_grad) and _only_numbers(res_k, res_v)
+                and _lib.current_device() == st.device.index):
             status = _lib.lib().pare_kivi_dense(
                 *st.cache_args(), *st.geometry(), st.n_comp,
-                full_k.data_ptr(), full_v.data_ptr(), _lib.dtype_code(st.dtype), full_k.stride(0), full_k.stride(1), full_k.stride(2),
-                st.res_k.data_ptr(), st.res_v.data_ptr(), st.res_k.stride(0), st.res_k.stride(1), st.res_k.stride(2), n_old,
-                *((left_k.data_ptr(), left_v.data_ptr(), left_k.stride(0), left_k.stride(1), left_k.stride(2),
-                   left_v.stride(0), left_v.stride(1), left_v.stride(2)) if n_left else (None, None, 0, 0, 0, 0, 0, 0)),
+                full_k.data_ptr(), full_v.data_ptr(), _lib.dtype_code(st.dtype), *full_k.stride()[:3],
+                *st.window_args(), n_old,
+                *((left_k.data_ptr(), left_v.data_ptr(), *left_k.stride()[:3], *left_v.stride()[:3]) if n_left
+                  else (None, None, 0, 0, 0, 0, 0, 0)),
                 n_left, stream)
         if status == 0:
             return full_k, full_v
@@ -406,8 +407,8 @@ class QuantizedKVCache:
                 full_k.stride(0), full_k.stride(1), full_k.stride(2), stream,
             )
             _lib.check(status, "pare_kivi_dequant")
-        full_k[:, :, st.n_comp:] = st.res_k[:, :, : st.r_len]
-        full_v[:, :, st.n_comp:] = st.res_v[:, :, : st.r_len]
+        full_k[:, :, st.n_comp:] = res_k[:, :, : st.r_len]
+        full_v[:, :, st.n_comp:] = res_v[:, :, : st.r_len]
         return full_k, full_v
 
     def attend(self, layer_idx: int, q: Tensor, new_k: Tensor, new_v: Tensor, scale: float | None = None,

@@ -311,7 +311,7 @@ def _stubbed_cache(monkeypatch, lib, shape=(1, 2, 128), dtype=torch.float16, **c
         t.fill_(-77.0)
     monkeypatch.setattr(_lib, "lib", lambda: lib)
     monkeypatch.setattr(_lib, "current_stream", lambda device: 0)
-    monkeypatch.setattr(torch.cuda, "current_device", lambda: None)      # the index of the stub store's device
+    monkeypatch.setattr(_lib, "current_device", lambda: None)            # the index of the stub store's device
     return cache
 
 
@@ -347,7 +347,7 @@ def test_update_of_what_no_kernel_takes(monkeypatch):
 
     lib = _CountingLib()
     cache = _stubbed_cache(monkeypatch, lib)
-    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    monkeypatch.setattr(_lib, "current_device", lambda: 1)
     got = cache.update(0, k.half(), v.half())
     assert torch.equal(got[0], k.half()) and torch.equal(got[1], v.half()) and lib.calls == []
 
