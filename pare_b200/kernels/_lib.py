@@ -150,9 +150,11 @@ def current_stream(device: torch.device) -> int:
 
 
 @functools.lru_cache(maxsize=1024)
-def w4a16_workspace_bytes(m: int, n: int, k: int, group_size: int) -> int:
-    """``pare_w4a16_workspace_bytes``: a function of the sizes alone, remembered for the shapes in use."""
-    return lib().pare_w4a16_workspace_bytes(m, n, k, group_size)
+def w4a16_workspace_bytes(m: int, n: int, k: int, group_size: int, index: int) -> int:
+    """``pare_w4a16_workspace_bytes`` on the CUDA device ``index``: a function of the sizes and of the device's number of
+    multiprocessors, remembered for the shapes in use."""
+    with torch.cuda.device(index):
+        return lib().pare_w4a16_workspace_bytes(m, n, k, group_size)
 
 
 # One zero-initialised workspace per device and stream; the kernels leave it zero-consistent.

@@ -89,7 +89,7 @@ def w4a16_forward(
         bias = bias.to(dtype)
     y = out if out is not None else torch.empty(m, n, device=dev, dtype=dtype)
     stream = _lib.current_stream(dev)
-    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size), stream)
+    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size, dev.index), stream)
     status = _lib.lib().pare_w4a16_forward(
         x.data_ptr(), code, x.stride(0),
         packed_weight.data_ptr(),
@@ -151,7 +151,7 @@ def w4a16_forward_prepared(prep: PreparedActivations, packed_weight: Tensor, sca
     y = out if out is not None else torch.empty(m, n, device=dev, dtype=prep.dtype)
     L = _lib.lib()
     stream = _lib.current_stream(dev)
-    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size), stream)
+    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size, dev.index), stream)
     if peer is not None:
         status = L.pare_w4a16_forward_prepared_allreduce(
             prep.data_ptr(), _lib.dtype_code(prep.dtype), packed_weight.data_ptr(),
@@ -195,7 +195,7 @@ def w4a16_forward_produced(producer: int, a: Tensor, packed_weight: Tensor, scal
     L = _lib.lib()
     dev = a.device
     stream = _lib.current_stream(dev)
-    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size), stream)
+    ws = _lib.workspace(dev, _lib.w4a16_workspace_bytes(m, n, k, group_size, dev.index), stream)
     if peer is not None:   # row-parallel shard: the sum over the ranks is added inside the kernel
         status = L.pare_w4a16_forward_produced_allreduce(
             producer, a.data_ptr(), _lib.ptr(delta), _lib.ptr(norm_weight), _lib.ptr(resid_out), a.stride(0), float(eps),

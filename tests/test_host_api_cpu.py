@@ -393,6 +393,31 @@ def test_outgrown_workspaces_stay_where_they_are(monkeypatch):
     assert _lib.workspace(cpu, 1, 8).numel() == 8 << 20
 
 
+def test_workspace_size_is_the_devices_own(monkeypatch):
+    """The plans behind the size depend on the number of multiprocessors: what is remembered for one device does not serve another."""
+    current = [0]
+
+    class Device:
+        def __init__(self, index):
+            self.index = index
+
+        def __enter__(self):
+            self.before, current[0] = current[0], self.index
+
+        def __exit__(self, *exc):
+            current[0] = self.before
+
+    class Lib:
+        def pare_w4a16_workspace_bytes(self, m, n, k, group_size):
+            return (m + n + k + group_size) * (1 + current[0])
+
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(_lib, "lib", lambda: Lib())
+    assert [_lib.w4a16_workspace_bytes(3, 16, 256, 128, index) for index in (0, 1, 0, 1)] == [403, 806, 403, 806]
+    assert current == [0]
+    _lib.w4a16_workspace_bytes.cache_clear()
+
+
 # ---- the C ABI ------------------------------------------------------------------------------------------
 
 def test_library_exports_every_declared_symbol():
