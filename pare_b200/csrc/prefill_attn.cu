@@ -681,7 +681,11 @@ extern "C" int pare_prefill_attn(const void* q, const void* k, const void* v, vo
   // described by a tensor map, and there is more than one 64-key tile (kernel alone, 32 query / 8 KV heads, bf16: 64 tokens
   // 9.0 us there, 6.6 us here; 128 tokens 10.3 / 9.5; 4 x 200 tokens 13.1 / 32.0; 512 tokens 18.5 / 33.9; 8192 tokens
   // 640 / 3250).  The kernel above serves the rest.
-  if (softmax_scale > 0.f && Tk > kPK) {
+  // Up to one key tile and query heads that share a KV head: two of them take turns on an SM there, 64-query tiles of all heads run
+  // at once here as long as there are SMs (128 tokens, batch 1 / 2 / 4 / 8: 10.5 / 10.6 / 10.8 / 11.3 there, 9.8 / 9.8 / 12.2 / 22.3 here;
+  // 8 heads that share nothing, batch 1: 8.4 / 9.5).
+  const bool all_at_once = Tk <= kTK && p.rep > 1 && (int64_t)((Tq + kPQ - 1) / kPQ) * Hq * B <= sm_count();
+  if (softmax_scale > 0.f && Tk > kPK && !all_at_once) {
     const int rc = prefill_tc(p, dtype, INT_MAX, tc::kWaitNs, s);
     if (rc != PARE_ERR_UNSUPPORTED) return rc;
   }
