@@ -340,8 +340,10 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid
   }
 }
 
-// Runs: equal shares of the units, or a few equal parts of each tile where that costs less adding up (microseconds: a
-// unit takes 0.65, a part about 0.25).
+// Runs: whole tiles, equal parts of a tile, or equal shares of all units (which cut tiles at odd places, so that a CTA finishes
+// two part tiles one after the other).  Microseconds, fitted to every run length of 19 heights x 10 depths with 8 and 16 rows: a unit
+// takes 0.575, a part 0.28, a cut tile 1.8, cuts at odd places 1.2 more (8192 x 4096, 8 rows: 128 CTAs of half a tile 9.9, 147 of
+// 7 units 11.1; 3072 x 4096: runs of 4 units 7.3, of 3 units 8.5; 14336 x 4096: whole tiles 12.8, runs of 13 units 14.6).
 TcPlan tc_plan(int N, int K) {
   TcPlan g{};
   g.tiles = (N + kRows - 1) / kRows;
@@ -351,8 +353,11 @@ TcPlan tc_plan(int N, int K) {
   double best = 1e30;
   auto consider = [&](int64_t run) {
     if (run < 1 || (units + run - 1) / run > sms) return;
-    const int64_t parts = run % g.ku ? (g.ku + run - 1) / run + 1 : 1;
-    const double cost = run * 0.65 + (parts > 1 ? 1.0 + 0.25 * parts : 0.0);
+    double cost = run * 0.575;
+    if (run % g.ku) {
+      const bool odd = g.ku % run != 0;
+      cost += (odd ? 3.0 : 1.8) + 0.28 * (double)((g.ku + run - 1) / run + odd);
+    }
     if (cost < best - 1e-9) {
       best = cost;
       g.run = (int)run;
