@@ -539,6 +539,7 @@ int launch_generic(const GemvParams& p, const uint8_t* packed, int G, cudaStream
 
 bool gemv_persist_supported(int M, int N, int K, int G, bool producer = false);
 size_t gemv_persist_partial_floats(int M, int N, int K);
+void gemv_persist_share(int M, int N, int K, int* whole, int* pieces);
 int gemv_persist_launch(const gemv::GemvParams& p, int x_dtype, cudaStream_t stream);
 bool gemv_tc_supported(int M, int N, int K, int G);
 size_t gemv_tc_partial_floats(int N, int K);
@@ -551,13 +552,24 @@ size_t prep_bytes(int M, int K) {  // prepared activations + step table, each ro
 }
 
 // Which calls go to the tensor core as codes (w4a16_gemv_tc.cu): its time hardly depends on the rows, the streaming kernels'
-// grows with them.  Microseconds there / here, bf16: 9 rows 28672 x 4096 23.5 / 32.3, 4096 x 14336 15.3 / 32.1, 4096 x 4096
-// 8.0 / 9.0; 8 rows 28672 x 4096 23.5 / 26.3, 6144 x 4096 10.3 / 10.6, 4096 x 4096 7.8 / 7.5; 5 rows 4096 x 14336 14.8 /
-// 16.0, 8192 x 28672 43 / 57, 28672 x 4096 23.1 / 22.1 (above 8192 columns the streaming kernels cut K into slices).
+// grows with them.  Microseconds there / here, bf16, kernels alone: 16 rows always (worst of 19 heights x 10 depths 5120 x 5120
+// 10.0 / 10.9), 9 rows 28672 x 4096 23.5 / 32.3, 4096 x 14336 15.3 / 32.1, 4096 x 4096 7.7 / 9.0.  8 rows: 6144 x 4096 9.3 / 10.5,
+// 28672 x 4096 18.9 / 21.5, 14336 x 4096 12.8 / 19.2, 8192 x 8192 15.0 / 23.1, 28672 x 2048 12.4 / 18.8, but 12288 x 4096 12.5 / 11.7
+// and 32768 x 4096 22.9 / 21.4 (streaming rounds that come out even), and below 24 Mi weights 3584 x 3584 8.1 / 7.0.  5 rows: 4096 x
+// 14336 14.8 / 16.0, 8192 x 28672 43 / 57, 28672 x 4096 23.1 / 22.1 (above 8192 columns the streaming kernels cut K into slices;
+// 1792 x 18944 15.2 / 14.3, where the heights are few the codes' CTAs are too).
 bool gemv_tc_rule(int M, int N, int K, int G) {
   if (!gemv_tc_supported(M, N, K, G)) return false;
-  const bool large = (int64_t)N * K >= (int64_t)24 << 20;
-  return M >= 9 || (M >= 7 && large) || (M >= 5 && large && K > 8192);
+  if (M >= 9) return true;
+  if ((int64_t)N * K < (int64_t)24 << 20) return false;
+  if (M < 7) return M >= 5 && K > 8192 && N >= 2048;
+  // Seven and eight rows.  One slice of 3072 - 4096 columns is what the streaming schedule is best at, and it gains on the codes with
+  // every round of whole tiles, but tiles left over are cut up where they are few, and adding the pieces takes 1 - 5 us.
+  if (K <= 3072 || K > 4096 || !gemv_persist_supported(M, N, K, G)) return true;
+  int whole, pieces;
+  gemv_persist_share(M, N, K, &whole, &pieces);
+  if (whole > 3) return pieces >= 8;
+  return whole == 3 || pieces > 1 || K <= 3584;
 }
 
 size_t gemv_workspace_bytes(int M, int N, int K, int G) {

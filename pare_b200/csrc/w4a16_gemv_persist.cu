@@ -606,6 +606,14 @@ bool gemv_persist_supported(int M, int N, int K, int G, bool producer) {
   return persist_smem(M, pl.sps, 2, pl.rows, pl.red_bufs) <= kPersistSmemCap;
 }
 
+// How the schedule shares out the 32-row tiles: whole tiles that every CTA takes, and pieces that each tile left over after that is cut
+// into (1: there are enough of them for most CTAs, or none).
+void gemv_persist_share(int M, int N, int K, int* whole, int* pieces) {
+  const StreamPlan pl = make_stream_plan(M, N, K);
+  *whole = pl.q;
+  *pieces = pl.P > 1 ? pl.P : 1;
+}
+
 // fp32 words of workspace behind the prepared activations: one [M][rows] block per contribution
 size_t gemv_persist_partial_floats(int M, int N, int K) {
   const StreamPlan pl = make_stream_plan(M, N, K);
