@@ -637,10 +637,18 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   // the outputs of the fused producers: a few KB from L2 per CTA instead of a launch of their own.  Not where many small
   // tiles would each do it, nor for the largest layers' three or four rows (one call, microseconds with / without the
   // launch: 4096 x 4096 1 row 6.5 / 5.1, 28672 x 4096 18.3 / 17.3, 3584 x 18944 15.0 / 13.3, 1024 x 4096 4 rows 7.6 / 6.8;
-  // 6144 x 4096, 384 tiles, 1 row 6.9 / 8.8; 57344 x 8192, 4 rows 77 / 80).
+  // 6144 x 4096, 384 tiles, 1 row 6.9 / 8.8; 57344 x 8192, 4 rows 77 / 80).  Nor where a CTA reads its activations in eight rounds,
+  // one after the other (4 rows of 3072 x 4096: 7.6 / 8.3, of 1024 x 5120 8.9 / 9.3, of 2048 x 8192 9.6 / 9.9).
   if (!prod && !prepared && !peer && M <= 4 && pl.fast && col_perm == nullptr && input_scale == nullptr && p.x_vec_ok) {
-    const bool few = gemv_persist_supported(M, N, K, G) ? M <= 2 || (int64_t)N * K <= (int64_t)1 << 27
-                                                        : (int64_t)((N + 16 * pl.rb - 1) / (16 * pl.rb)) * pl.splits <= 2 * sm_count();
+    bool few;
+    if (gemv_persist_supported(M, N, K, G)) {
+      int whole, pieces;
+      gemv_persist_share(M, N, K, &whole, &pieces);
+      few = M <= 2 || ((int64_t)N * K <= (int64_t)1 << 27 && (M == 3 || whole > 0));
+    } else {
+      const int rounds = (pl.steps_per_split + 2 * pl.warps - 1) / (2 * pl.warps);   // per row: a half warp takes a step
+      few = (int64_t)((N + 16 * pl.rb - 1) / (16 * pl.rb)) * pl.splits <= 2 * sm_count() && M * rounds <= 6;
+    }
     if (few) {
       p.producer = kProducerPlain;
       p.pa = x;
