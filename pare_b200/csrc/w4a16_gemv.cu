@@ -639,7 +639,11 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   // launch: 4096 x 4096 1 row 6.5 / 5.1, 28672 x 4096 18.3 / 17.3, 3584 x 18944 15.0 / 13.3, 1024 x 4096 4 rows 7.6 / 6.8;
   // 6144 x 4096, 384 tiles, 1 row 6.9 / 8.8; 57344 x 8192, 4 rows 77 / 80).  Nor where a CTA reads its activations in eight rounds,
   // one after the other (4 rows of 3072 x 4096: 7.6 / 8.3, of 1024 x 5120 8.9 / 9.3, of 2048 x 8192 9.6 / 9.9).
-  if (!prod && !prepared && !peer && M <= 4 && pl.fast && col_perm == nullptr && input_scale == nullptr && p.x_vec_ok) {
+  // Nor where the output is written over the activations: every CTA of the streaming kernel would read rows that others already write.
+  const auto* const xb = reinterpret_cast<const unsigned char*>(x);
+  const auto* const yb = reinterpret_cast<const unsigned char*>(y);
+  const bool apart = xb + ((int64_t)(M - 1) * ldx + K) * 2 <= yb || yb + ((int64_t)(M - 1) * ldy + N) * 2 <= xb;
+  if (!prod && !prepared && !peer && M <= 4 && pl.fast && col_perm == nullptr && input_scale == nullptr && p.x_vec_ok && apart) {
     bool few;
     if (gemv_persist_supported(M, N, K, G)) {
       int whole, pieces;

@@ -27,3 +27,20 @@ def test_same_bits_as_prepared_activations(n, k, m, dtype, cuda_lib):
     sc, ze = layer.scale.squeeze(-1).contiguous(), layer.zero.squeeze(-1).contiguous()
     perm = torch.arange(k, device="cuda", dtype=torch.int32)
     assert torch.equal(w4a16_forward(x.contiguous(), layer.packed_weight, sc, ze, 128, col_perm=perm), want)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 8, 16])
+@pytest.mark.parametrize("n", [256, 2048, 4096, 8192])
+def test_output_over_the_activations(n, m, cuda_lib):
+    """``out`` may be the activations themselves, or overlap them: they are read before anything is written."""
+    layer = synthetic_linear(n, n, seed=n, device="cuda")
+    sc, ze = layer.scale.squeeze(-1).contiguous(), layer.zero.squeeze(-1).contiguous()
+    x = torch.randn(m, n, device="cuda", generator=torch.Generator("cuda").manual_seed(m)).half()
+    want = layer(x)
+    for shift in (0, 8, n // 2):                 # out starts `shift` elements into the activations
+        for _ in range(5):
+            buf = torch.zeros(m * n + shift, device="cuda", dtype=torch.float16)
+            a, out = buf[: m * n].view(m, n), buf[shift:].view(m, n)
+            a.copy_(x)
+            w4a16_forward(a, layer.packed_weight, sc, ze, 128, out=out)
+            assert torch.equal(out, want)
