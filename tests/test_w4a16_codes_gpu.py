@@ -9,7 +9,7 @@ import torch
 
 from pare_b200.decode import synthetic_linear
 from pare_b200.kernels import _lib
-from pare_b200.kernels.matmul_int4 import prepare
+from pare_b200.kernels.matmul_int4 import prepare, w4a16_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -75,3 +75,23 @@ def test_cold_weights_many_units(cuda_lib):
     for _ in range(4):
         flush.zero_()
         assert torch.equal(layer(xl), first)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("act_order", [False, True])
+@pytest.mark.parametrize("n,k,m", [(129, 768, 9), (640, 4096, 16), (2048, 14336, 6), (6144, 4096, 8)])
+def test_bias_input_scale_and_act_order(n, k, m, act_order, dtype, cuda_lib):
+    """What the preparation launch does (quotient by a run-time scale rounded to the dtype, gather) and what the fold adds."""
+    g = torch.Generator("cuda").manual_seed(n + m)
+    layer = synthetic_linear(n, k, seed=n, device="cuda")
+    scale_in = torch.exp(0.5 * torch.randn(k, device="cuda", generator=g))
+    bias = torch.randn(n, device="cuda", generator=g).to(dtype)
+    perm = torch.randperm(k, device="cuda", generator=g).to(torch.int32) if act_order else None
+    x = torch.randn(m, k, device="cuda", generator=g).to(dtype)
+    y = w4a16_forward(x, layer.packed_weight, layer.scale.squeeze(-1).contiguous(), layer.zero.squeeze(-1).contiguous(), 128, bias=bias,
+                      col_perm=perm, input_scale=scale_in)
+    xs = (x.float() / scale_in).to(dtype)
+    ref, mag = _layer_reference(layer, xs[:, perm.long()] if act_order else xs)
+    ref = ref + bias.double()
+    ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert bool(((y.double() - ref).abs() <= ulp * ref.abs() + k * 2.0 ** -23 * mag + 1e-7).all())
