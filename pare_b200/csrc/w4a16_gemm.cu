@@ -23,8 +23,8 @@
 // two-wide fp32 instructions, codes read in place as subnormal floats: dequant_word below) and rounds to the 16-bit
 // type.  Weights therefore reach the tensor core as exactly dtype(fp32((q - zero) * scale)),
 // bit for bit what the reference's own dequantize-then-matmul path feeds its GEMM (pare/layers/linear.py:112-118, 129).
-// All mbarrier waits are bounded; on expiry the CTA records PARE_ERR_TIMEOUT, stops waiting,
-// frees its tensor memory and returns.
+// All mbarrier waits are bounded; on expiry the CTA records PARE_ERR_TIMEOUT, stops waiting and loading, lets its copies and
+// products in flight end (bounded again), frees its tensor memory and returns.
 
 #include "tcgen05.cuh"
 
@@ -174,9 +174,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
   const int stages = p.stages, rstages = p.raw_stages;
   const uint32_t b_ring = s_u32(smem), raw = b_ring + stages * b_stage;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + stages * b_stage + rstages * kRawBytes);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxRaw + 2 * kMaxStages + 4);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxRaw + 2 * kMaxStages + 5);
   const uint32_t raw_full = s_u32(bars), raw_empty = raw_full + kMaxRaw * 8, ab_full = raw_empty + kMaxRaw * 8,
-                 ab_empty = ab_full + kMaxStages * 8, acc_full = ab_empty + kMaxStages * 8, acc_empty = acc_full + 16;
+                 ab_empty = ab_full + kMaxStages * 8, acc_full = ab_empty + kMaxStages * 8, acc_empty = acc_full + 16, mma_done = acc_empty + 16;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform, and known to be
   const int ku = p.tile_units;
@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
       bar_init(ab_full + i * 8, kDequantThreads / 32 + 1);
       bar_init(ab_empty + i * 8, 1);
     }
+    bar_init(mma_done, 1);
     for (int i = 0; i < 2; ++i) {
       bar_init(acc_full + i * 8, 1);
       bar_init(acc_empty + i * 8, 4);
@@ -281,32 +282,38 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
   } else if (warp == 8) {
     // ================= packed codes =================
     if (lane == 0) {
-      int slot = 0;
+      int slot = 0, u = u0;
       uint32_t par = 1;
-      for (int u = u0; u < u1; ++u) {
+      for (; u < u1; ++u) {
         const int t = u / ku, k = u - t * ku;
         bar_wait(raw_empty + slot * 8, par, status, dead);
+        if (dead) break;
         bar_expect(raw_full + slot * 8, kRawBytes);
         tma_tile(raw + slot * kRawBytes, &tm_w, k * (kUnitK / 2), row_tile(t) * kRows, raw_full + slot * 8);
         if (++slot == rstages) slot = 0, par ^= 1;
       }
+      bool late = false;
+      for (int j = max(0, u - u0 - rstages); j < u - u0; ++j) bar_wait(raw_full + (j % rstages) * 8, (j / rstages) & 1, status, late);
     }
     __syncwarp();
   } else if (warp == 9) {
     // ================= activations =================
     if (lane == 0) {
-      int s = 0;
+      int s = 0, issued = 0;
       uint32_t par = 1;
-      for (int u = u0; u < u1; ++u) {
+      for (int u = u0; u < u1 && !dead; ++u) {
         const int t = u / ku, k = u - t * ku, m0 = act_tile(t) * p.mt;
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 2; ++j, ++issued) {
           bar_wait(ab_empty + s * 8, par, status, dead);
+          if (dead) break;
           bar_expect(ab_full + s * 8, b_stage);
           tma_tile(b_ring + s * b_stage, &tm_x, k * kUnitK + j * kStageK, m0, ab_full + s * 8);
           tma_tile(b_ring + s * b_stage + b_blk, &tm_x, k * kUnitK + j * kStageK + kBlockK, m0, ab_full + s * 8);
           if (++s == stages) s = 0, par ^= 1;
         }
       }
+      bool late = false;
+      for (int i = max(0, issued - stages); i < issued; ++i) bar_wait(ab_full + (i % stages) * 8, (i / stages) & 1, status, late);
     }
     __syncwarp();
   } else if (warp == 10) {
@@ -337,6 +344,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __gri
       umma_commit(acc_full + buf * 8, me);
       u += nst / 2;
     }
+    umma_commit(mma_done, me);
+    bool late = false;
+    bar_wait(mma_done, 0, status, late);
     __syncwarp();
   } else if (warp >= 12) {
     // ================= epilogue: tensor memory -> registers -> global =================

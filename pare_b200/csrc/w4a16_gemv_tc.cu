@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t raw = s_u32(smem), b_ring = raw + kRaw * kRawBytes, bars = b_ring + kStages * kBStage;
   const uint32_t raw_full = bars, raw_empty = raw_full + kRaw * 8, ab_full = raw_empty + kRaw * 8, ab_empty = ab_full + kStages * 8,
-                 d_full = ab_empty + kStages * 8, d_empty = d_full + kSums * 8, tmem_slot = d_empty + kSums * 8;
+                 d_full = ab_empty + kStages * 8, d_empty = d_full + kSums * 8, mma_done = d_empty + kSums * 8, tmem_slot = mma_done + 8;
   float* xchg = reinterpret_cast<float*>(smem + kRaw * kRawBytes + kStages * kBStage + 512);   // [kN][kRows]
   // (SX, g) of every step and activation row
   float2* tab = reinterpret_cast<float2*>(smem + kRaw * kRawBytes + kStages * kBStage + 512 + kXchg);
@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid
   pdl_launch_dependents();
 
   if (threadIdx.x == 0) {
+    bar_init(mma_done, 1);
     for (int i = 0; i < kRaw; ++i) {
       bar_init(raw_full + i * 8, 1);
       bar_init(raw_empty + i * 8, 8);
@@ -152,10 +153,12 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid
     int slot = 0;
     uint32_t par = 1;
     const int upl = max(1, 8 * p.steps_per_group / 2);   // units per 32-byte sector of a scale row
-    for (int u = u0; u < u1; ++u) {
+    int u = u0;
+    for (; u < u1; ++u) {
       const int t = u / ku, k = u - t * ku;
+      if (lane == 0) bar_wait(raw_empty + slot * 8, par, status, dead);
+      if (__any_sync(0xffffffffu, dead)) break;
       if (lane == 0) {
-        bar_wait(raw_empty + slot * 8, par, status, dead);
         bar_expect(raw_full + slot * 8, kRawBytes);
         tma_tile(raw + slot * kRawBytes, &tm_w, k * (kUnitK / 2), t * kRows, raw_full + slot * 8);
       }
@@ -171,22 +174,30 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid
       }
       if (++slot == kRaw) slot = 0, par ^= 1;
     }
+    if (lane == 0) {   // the block may end only when what it asked for has arrived, also where a wait ran out
+      bool late = false;
+      for (int j = max(0, u - u0 - kRaw); j < u - u0; ++j) bar_wait(raw_full + (j % kRaw) * 8, (j / kRaw) & 1, status, late);
+    }
+    __syncwarp();
   } else if (warp == 9) {
     // ================= activations =================
     if (lane == 0) {
       pdl_wait();
-      int s = 0;
+      int s = 0, issued = 0;
       uint32_t par = 1;
-      for (int u = u0; u < u1; ++u) {
+      for (int u = u0; u < u1 && !dead; ++u) {
         const int k = u % ku;
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 2; ++j, ++issued) {
           bar_wait(ab_empty + s * 8, par, status, dead);
+          if (dead) break;
           bar_expect(ab_full + s * 8, kBStage);
           tma_tile(b_ring + s * kBStage, &tm_x, k * kUnitK + j * 128, 0, ab_full + s * 8);
           tma_tile(b_ring + s * kBStage + kBBlk, &tm_x, k * kUnitK + j * 128 + 64, 0, ab_full + s * 8);
           if (++s == kStages) s = 0, par ^= 1;
         }
       }
+      bool late = false;
+      for (int i = max(0, issued - kStages); i < issued; ++i) bar_wait(ab_full + (i % kStages) * 8, (i / kStages) & 1, status, late);
     }
     __syncwarp();
   } else if (warp == 10) {
@@ -210,6 +221,9 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid
       if (++s == kStages) s = 0, par ^= 1;
       if (++d == kSums) d = 0, dpar ^= 1;
     }
+    umma_commit(mma_done, me);
+    bool late = false;
+    bar_wait(mma_done, 0, status, late);
     __syncwarp();
   } else if (warp >= 12) {
     // ================= fold and output =================
