@@ -12,7 +12,6 @@ namespace pare {
 namespace gemv {
 
 constexpr int kProducerPlain = 16;   // activations as they are (a = x [M][lda], no gather, no input scale): only brought into operand order
-constexpr int kStageRounds = 4;   // most steps a half warp of the staging threads takes: K <= 128 * rounds * threads / 16
 
 // Norm weights of the steps a thread will produce: constants of the model, so they can be fetched before
 // the dependency wait.  ROUNDS as in stage_produce.

@@ -1,4 +1,4 @@
-// Shared pieces of the tensor-memory kernels (w4a16_gemm.cu, prefill_attn.cu): mbarriers with bounded waits, tensor-map
+// Shared pieces of the tensor-memory kernels (w4a16_gemm.cu, w4a16_gemv_tc.cu, prefill_attn.cu): mbarriers with bounded waits, tensor-map
 // copies, tcgen05 descriptors and instructions.
 #pragma once
 
@@ -87,7 +87,6 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
   return (uint64_t)((smem_addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
          ((uint64_t)2 << 61);
 }
-// A (weights) in tensor memory: 128 lanes x 8 columns of two 16-bit elements per instruction
 // The issuing warp runs its loop with all lanes and only these instructions under the elected lane's predicate: in a
 // one-lane branch the operands are not known to be uniform, and every instruction is preceded by moves of its descriptors
 // into uniform registers (about 65 cycles apiece, which paced the kernels at few activation rows).
@@ -100,6 +99,7 @@ __device__ __forceinline__ uint32_t elect_one() {
       : "=r"(e));
   return e;
 }
+// A (weights) in tensor memory: 128 lanes x 8 columns of two 16-bit elements per instruction
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"

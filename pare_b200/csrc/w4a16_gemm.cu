@@ -7,8 +7,9 @@
 // every instruction:   Y^T[n][m] = sum_k W[n][k] * X[m][k].
 //
 // A persistent grid, one CTA per SM.  The work is the list of (128-row weight tile, activation tile, 256-column unit)
-// in that nesting order (the first two exchanged for very large activations); a CTA takes one contiguous run of units, so a run may begin and end inside a tile.  Tiles that
-// lie in several runs are finished by the CTA that arrives last, which adds the fp32 partial sums in K order.
+// in that nesting order (the first two exchanged for very large activations); a CTA takes one contiguous run of units, so a
+// run may begin and end inside a tile.  Tiles that lie in several runs are finished by the CTA that arrives last, which adds
+// the fp32 partial sums in K order.
 // Warp roles:
 //   warps 0-7    dequantize (two groups of four warps, one per 64-column block of a 128-column stage, one thread per
 //                weight row): codes from shared memory, 16-bit weights into TENSOR MEMORY (tcgen05.st), where the MMA
@@ -40,7 +41,6 @@ constexpr int kUnitK = 256;            // columns per unit of work: one tensor-m
 constexpr int kRawBytes = kRows * 128; // bytes of a unit's codes: 128 rows x 128 bytes, 128B swizzle
 constexpr int kMaxStages = 4;          // operand stages: 4 x 64 tensor-memory columns of weights beside the accumulators
 constexpr int kMaxRaw = 8;
-constexpr int kMaxMt = 256;            // activation rows per tile (UMMA N)
 constexpr uint32_t kTmemCols = 512;    // accumulators: columns 0-255 (two of up to 128, or one of up to 256)
 constexpr uint32_t kTmemA = 256;       // weights: columns 256-511
 constexpr int kDequantThreads = 256;
@@ -50,13 +50,12 @@ constexpr size_t kCounterBytes = kCounterInts * sizeof(int);
 constexpr size_t kStatusIndex = kCounterInts - 1;
 
 struct GemmParams {
-  const uint8_t* packed;
   const float* scale;
   const float* zero;
   const void* bias;
   void* y;
   int64_t ldy;
-  int M, N, K, ngroups, group_size;
+  int M, N, ngroups, group_size;
   int mt;               // activation rows per tile (UMMA N): a multiple of 16, 32 .. 256
   int inner;            // tiles of the inner direction of the tile order
   int rows_inner;       // 1: weight tiles are the inner direction (activation tiles the outer), 0: the other way round
@@ -632,7 +631,6 @@ int gemm_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
                PARE_ERR_CUDA);
 
   GemmParams p{};
-  p.packed = packed;
   p.scale = scale;
   p.zero = zero;
   p.bias = bias;
@@ -640,7 +638,6 @@ int gemm_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   p.ldy = ldy;
   p.M = M;
   p.N = N;
-  p.K = K;
   p.ngroups = K / G;
   p.group_size = G;
   p.mt = g.mt;
