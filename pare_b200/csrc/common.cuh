@@ -22,20 +22,29 @@ inline int launch_status() { return cudaGetLastError() == cudaSuccess ? PARE_OK 
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Streaming multiprocessors of the current device (cached per device; 148 on a B200).  Schedules are sized by it;
-// nothing depends on it for correctness.
-inline int sm_count() {
+// An attribute of the current device (cached per device by the caller's `cached`).  Schedules are sized by these;
+// nothing depends on them for correctness.
+inline int device_attribute(cudaDeviceAttr attr, int (&cached)[64], int otherwise) {
   static std::mutex mu;
-  static int cached[64] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return otherwise;
   std::lock_guard<std::mutex> lock(mu);
   if (cached[dev] == 0) {
     int v = 0;
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+    if (cudaDeviceGetAttribute(&v, attr, dev) != cudaSuccess || v <= 0) v = otherwise;
     cached[dev] = v;
   }
   return cached[dev];
+}
+// Streaming multiprocessors (148 on a B200)
+inline int sm_count() {
+  static int cached[64] = {};
+  return device_attribute(cudaDevAttrMultiProcessorCount, cached, 148);
+}
+// Bytes of L2 (126 MB on a B200)
+inline int l2_bytes() {
+  static int cached[64] = {};
+  return device_attribute(cudaDevAttrL2CacheSize, cached, 126 << 20);
 }
 
 // cudaFuncSetAttribute(max dynamic shared memory) once per (kernel, device), thread-safe.  Keyed by the kernel's

@@ -561,7 +561,7 @@ GemmPlan gemm_plan(int M, int N, int K) {
   // by themselves, smaller activations stay in L2 (28672 x 4096, 1531 rows: 293 us, 309 the other way), and codes larger than
   // the activations would be the ones re-read (57344 x 8192, 1000 rows: 1052 / 1418 us).
   const double act = 2.0 * M * K, codes = 0.5 * N * K;
-  g.rows_inner = g.split && act > 126e6 && codes < act;
+  g.rows_inner = g.split && act > (double)l2_bytes() && codes < act;
   return g;
 }
 
