@@ -102,3 +102,32 @@ def test_a_wait_that_runs_out_gives_nan(hq, h, t, loads, cuda_lib):
     assert bool(torch.isnan(out[:, :, whole:]).all())
     assert bool((torch.isnan(out[:, :, :whole]) | (out[:, :, :whole] == want[:, :, :whole])).all())
     assert torch.equal(prefill_attention(q, k, v), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("hq,h", [(1, 1), (2, 1), (3, 1)])
+@pytest.mark.parametrize("tq,tk", [(300, 300), (129, 256), (200, 520), (640, 641)])
+def test_values_of_hidden_keys_do_not_matter(hq, h, tq, tk, dtype, cuda_lib):
+    """An infinity or a NaN among the values reaches the queries that see its key, in its channel, and nothing else: the channel of the
+    queries before it is what it is with a zero in that place (to the bound of the length tests: it is summed again), every other
+    output keeps its bits."""
+    g = torch.Generator("cuda").manual_seed(tk)
+    q = torch.randn(2, hq, tq, 128, device="cuda", generator=g).to(dtype)
+    k = torch.randn(2, h, tk, 128, device="cuda", generator=g).to(dtype)
+    v = torch.randn(2, h, tk, 128, device="cuda", generator=g).to(dtype)
+    ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    off = tk - tq
+    for key, channel, bad in ((off + 1, 3, "nan"), (off + 63, 64, "inf"), (off + 64, 127, "-inf"), (off + 100, 0, "nan"), (off + 127, 70, "inf"),
+                              (min(off + 128, tk - 1), 9, "inf"), (tk - 1, 33, "nan"), (tk - 1, 96, "-inf"), (0, 5, "inf")):
+        w = v.clone()
+        w[0, 0, key, channel] = 0.0
+        want = prefill_attention(q, k, w)
+        w[0, 0, key, channel] = float(bad)
+        out = prefill_attention(q, k, w)
+        share = slice(0, hq // h)                         # the query heads of that KV head, in the first sequence only
+        first = max(0, key - off)                         # the first query that sees the key
+        assert bool((~torch.isfinite(out[0, share, first:, channel])).all()), key
+        before, ref = out[0, share, :first, channel].double(), want[0, share, :first, channel].double()
+        assert bool(((before - ref).abs() <= 2 * ulp * ref.abs() + 2.0 ** -13).all()), key
+        out[0, share, :, channel] = want[0, share, :, channel]
+        assert torch.equal(out, want), key
