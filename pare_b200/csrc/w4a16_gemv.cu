@@ -646,9 +646,12 @@ int gemv_forward(const void* x, int x_dtype, int64_t ldx, const uint8_t* packed,
   if (!prod && !prepared && !peer && M <= 4 && pl.fast && col_perm == nullptr && input_scale == nullptr && p.x_vec_ok && apart) {
     bool few;
     if (gemv_persist_supported(M, N, K, G)) {
-      int whole, pieces;
-      gemv_persist_share(M, N, K, &whole, &pieces);
-      few = M <= 2 || ((int64_t)N * K <= (int64_t)1 << 27 && (M == 3 || whole > 0));
+      few = M <= 2 || (int64_t)N * K <= (int64_t)1 << 27;
+      if (few && M == 4) {
+        int whole, pieces;
+        gemv_persist_share(M, N, K, &whole, &pieces);
+        few = whole > 0;
+      }
     } else {
       const int rounds = (pl.steps_per_split + 2 * pl.warps - 1) / (2 * pl.warps);   // per row: a half warp takes a step
       few = (int64_t)((N + 16 * pl.rb - 1) / (16 * pl.rb)) * pl.splits <= 2 * sm_count() && M * rounds <= 6;

@@ -159,10 +159,10 @@ class QuantizedLinear(nn.Module):
         return bufs
 
     def _forward_kernel(self, x: Tensor) -> Tensor:
-        bufs = self._kernel_buffers()
-        dtype, flat = x.dtype, x.dim() == 2 and x.shape[1] == self.in_features   # else the last reshape refuses what does not fit
+        bufs, k, shape, dtype = self._kernel_buffers(), self.in_features, x.shape, x.dtype
+        flat = len(shape) == 2 and shape[1] == k   # else the last reshape refuses what does not fit
         # reshape also gives a single row (a slice of padded or broadcast rows) a pitch of its own
-        x2d = x if flat and (x.stride(0) == self.in_features or x.shape[0] > 1) else x.reshape(-1, self.in_features)
+        x2d = x if flat and (shape[0] > 1 or x.stride(0) == k) else x.reshape(-1, k)
         if dtype is not torch.float16 and dtype is not torch.bfloat16:
             x2d = x2d.to(torch.float16)
         if x2d.stride(1) != 1:
@@ -176,12 +176,12 @@ class QuantizedLinear(nn.Module):
             self._kernel_group_size(),
             bias=self.bias,
             col_perm=bufs["_col_perm_kernel"],
-            input_scale=self.input_scale,
+            input_scale=bufs["input_scale"],
             meta_h2=bufs["_meta_h2_kernel"] if use_h2 else None,
         )
         if y.dtype is not dtype:
             y = y.to(dtype)
-        return y if flat else y.reshape(*x.shape[:-1], self.out_features)
+        return y if flat else y.reshape(*shape[:-1], self.out_features)
 
     def supports_prepared(self, rows: int) -> bool:
         """True if :meth:`forward_prepared` can serve ``rows`` activation rows of this layer."""
