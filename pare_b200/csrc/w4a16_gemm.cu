@@ -161,8 +161,8 @@ __device__ __forceinline__ void dequant_word(uint32_t w, const DqConst& c, uint3
 // times what it moves in the 1024 cycles of the MMAs.  With the weights in tensor memory 144 KB remain, and the freed 64 KB
 // hold one more activation stage.  Few rows are bound by the dequantizing warps (about 750 cycles per 128 columns);
 // four stages instead of two keep the MMA's round trip off their path, and equal runs of units instead of whole tiles per
-// CTA keep all SMs busy to the end.  28672 x 4096: 64 rows 65.9 -> 36.6 us, 256 rows 74.5 -> 59.4, 2048 rows 473 -> 395 us
-// (1217 TFLOP/s); 4096 x 4096: 64 rows 23.6 -> 14.9, 128 rows 35.0 -> 17.2; 3584 x 18944, 1531 rows 294 -> 188 us.
+// CTA keep all SMs busy to the end.  28672 x 4096: 64 rows 65.9 -> 33.7 us, 256 rows 74.5 -> 52.7, 2048 rows 473 -> 356 us
+// (1350 TFLOP/s); 4096 x 4096: 64 rows 23.6 -> 13.6, 128 rows 35.0 -> 16.2; 3584 x 18944, 1531 rows 294 -> 182 us.
 template <typename T>
 __global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                                                                     const GemmParams p) {
@@ -506,11 +506,11 @@ struct GemmPlan {
 
 // Heights of the activation tiles (a multiple of 16, what the MMA's N takes, all tiles alike) and runs (a CTA's share in
 // units of 256 columns) by a cost in microseconds, fitted to a sweep over 32 - 512 rows, 4096 / 6144 / 28672 x 4096 and
-// 4096 x 14336 (bf16): a unit takes 1.07 at 32 rows and 1.3 - 1.6 at 256, so tall tiles win once they fill the SMs; below
-// that, more tiles of fewer rows beat cutting K (4096 x 4096, 128 rows: 64 tiles of 64 rows in two parts 19.4, 32 tiles of
-// 128 rows in four parts 23.4; 512 rows: 128 tiles of 128 rows 25.9, 64 of 256 in two parts 36).  A tile above 128 rows
-// has a single accumulator, so its epilogue stalls the next tile's products.  Parts are written and read again by one CTA
-// (about 14 ns per row and part), more of them where a run does not end with its tile.
+// 4096 x 14336 (bf16), with an epilogue that took longer than the present one: a unit takes 1.0 at 32 - 128 rows and 1.5 - 1.7 at
+// 256, so tall tiles win once they fill the SMs; below that, more tiles of fewer rows beat cutting K (4096 x 4096, 128 rows: 64
+// tiles of 64 rows in two parts 16.9, 32 tiles of 128 rows in four parts 17.9; 512 rows: 128 tiles of 128 rows 21.3, 64 of 256
+// in two parts 26.6).  A tile above 128 rows has a single accumulator, so its epilogue stalls the next tile's products.  Parts are
+// written and read again by one CTA (about 14 ns per row and part), more of them where a run does not end with its tile.
 GemmPlan gemm_plan(int M, int N, int K) {
   GemmPlan best_plan{};
   double best = 1e30;
@@ -557,8 +557,8 @@ GemmPlan gemm_plan(int M, int N, int K) {
   // Tile order.  Activation tiles inner: a CTA stays with its weight rows, codes are read once.  When runs cut tiles, the CTAs are
   // at different depths of different activation tiles, and activations that do not fit L2 then come from DRAM over and over
   // (4999 x 14336 for 4096 rows: 4.6 GB in 600 us); with the weight tiles inner, neighbouring CTAs walk the same activation
-  // tile together: 636 -> 531 us, 8192 x 28672 with 3000 / 4999 rows 1545 / 2879 -> 1252 / 2246 us.  Whole tiles per CTA keep step
-  // by themselves, smaller activations stay in L2 (28672 x 4096, 1531 rows: 293 us, 309 the other way), and codes larger than
+  // tile together (measured with the epilogue before the present one): 636 -> 531 us, 8192 x 28672 with 3000 / 4999 rows 1545 / 2879
+  // -> 1252 / 2246 us.  Whole tiles per CTA keep step by themselves, smaller activations stay in L2 (28672 x 4096, 1531 rows: 293 us, 309 the other way), and codes larger than
   // the activations would be the ones re-read (57344 x 8192, 1000 rows: 1052 / 1418 us).
   const double act = 2.0 * M * K, codes = 0.5 * N * K;
   g.rows_inner = g.split && act > (double)l2_bytes() && codes < act;

@@ -552,12 +552,12 @@ size_t prep_bytes(int M, int K) {  // prepared activations + step table, each ro
 }
 
 // Which calls go to the tensor core as codes (w4a16_gemv_tc.cu): its time hardly depends on the rows, the streaming kernels'
-// grows with them.  Microseconds there / here, bf16, kernels alone: 16 rows always (worst of 19 heights x 10 depths 5120 x 5120
-// 10.0 / 10.9), 9 rows 28672 x 4096 23.5 / 32.3, 4096 x 14336 15.3 / 32.1, 4096 x 4096 7.7 / 9.0.  8 rows: 6144 x 4096 9.3 / 10.5,
-// 28672 x 4096 18.9 / 21.5, 14336 x 4096 12.8 / 19.2, 8192 x 8192 15.0 / 23.1, 28672 x 2048 12.4 / 18.8, but 12288 x 4096 12.5 / 11.7
-// and 32768 x 4096 22.9 / 21.4 (streaming rounds that come out even), and below 24 Mi weights 3584 x 3584 8.1 / 7.0.  5 rows: 4096 x
-// 14336 14.8 / 16.0, 8192 x 28672 43 / 57, 28672 x 4096 23.1 / 22.1 (above 8192 columns the streaming kernels cut K into slices;
-// 1792 x 18944 15.2 / 14.3, where the heights are few the codes' CTAs are too).
+// grows with them.  Microseconds there / here, bf16, kernels alone: 16 rows always (closest of 19 heights x 10 depths: 3584 x 3584
+// 8.5 / 10.2), 9 rows 28672 x 4096 23.1 / 32.3, 4096 x 14336 13.7 / 32.1, 4096 x 4096 7.8 / 9.0.  8 rows: 6144 x 4096 9.3 / 10.5,
+// 28672 x 4096 22.7 / 25.7, 14336 x 4096 12.8 / 19.2, 8192 x 8192 14.7 / 22.7, 28672 x 2048 12.4 / 18.8, but 12288 x 4096 12.5 / 11.7
+// and 32768 x 4096 22.9 / 21.4 (streaming rounds that come out even), and below 24 Mi weights 3584 x 3584 8.2 / 7.1.  5 rows: 4096 x
+// 14336 13.5 / 16.0, 8192 x 28672 43 / 57, 28672 x 4096 22.0 / 22.1 (above 8192 columns the streaming kernels cut K into slices;
+// 1792 x 18944 15.2 / 14.3 a call: where the heights are few the codes' CTAs are too).
 bool gemv_tc_rule(int M, int N, int K, int G) {
   if (!gemv_tc_supported(M, N, K, G)) return false;
   if (M >= 9) return true;

@@ -52,9 +52,9 @@ struct TcArgs {
 };
 
 // What bounds it (one B200, bf16, kernel alone): the codes arrive at 4.7 TB/s when nothing else is done (12.4 us for 28672 x
-// 4096), the unpack - multiply - fold chain of a 256-column unit takes 0.65 us of an SM, and 5 - 6 us are launch, first
-// loads and drain.  16 rows: 28672 x 4096 40.2 -> 23.9 us, 4096 x 14336 34.9 -> 15.6, 4096 x 4096 11.0 -> 8.3,
-// 57344 x 8192 322 -> 73, 8192 x 28672 242 -> 44 us against the streaming kernels, whose activations (16 rows x 4096
+// 4096), the unpack - multiply - fold chain of a 256-column unit takes 0.6 us of an SM, and 5 - 6 us are launch, first
+// loads and drain.  16 rows: 28672 x 4096 40.2 -> 23.7 us, 4096 x 14336 34.9 -> 13.9, 4096 x 4096 11.0 -> 7.8,
+// 57344 x 8192 322 -> 73, 8192 x 28672 242 -> 45 us against the streaming kernels, whose activations (16 rows x 4096
 // columns) fill shared memory and whose warp-level operand handling grows with the rows.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1) w4a16_gemv_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
