@@ -557,9 +557,10 @@ GemmPlan gemm_plan(int M, int N, int K) {
   // Tile order.  Activation tiles inner: a CTA stays with its weight rows, codes are read once.  When runs cut tiles, the CTAs are
   // at different depths of different activation tiles, and activations that do not fit L2 then come from DRAM over and over
   // (4999 x 14336 for 4096 rows: 4.6 GB in 600 us); with the weight tiles inner, neighbouring CTAs walk the same activation
-  // tile together (measured with the epilogue before the present one): 636 -> 531 us, 8192 x 28672 with 3000 / 4999 rows 1545 / 2879
-  // -> 1252 / 2246 us.  Whole tiles per CTA keep step by themselves, smaller activations stay in L2 (28672 x 4096, 1531 rows: 293 us, 309 the other way), and codes larger than
-  // the activations would be the ones re-read (57344 x 8192, 1000 rows: 1052 / 1418 us).
+  // tile together (measured with the epilogue before the present one): 636 -> 531 us, 8192 x 28672 with 3000 / 4999 rows
+  // 1545 / 2879 -> 1252 / 2246 us.  Whole tiles per CTA keep step by themselves, smaller activations stay in L2 (28672 x 4096,
+  // 1531 rows: 293 us, 309 the other way), and codes larger than the activations would be the ones re-read (57344 x 8192,
+  // 1000 rows: 1052 / 1418 us).
   const double act = 2.0 * M * K, codes = 0.5 * N * K;
   g.rows_inner = g.split && act > (double)l2_bytes() && codes < act;
   return g;
